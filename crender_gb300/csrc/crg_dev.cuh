@@ -104,11 +104,15 @@ __device__ __forceinline__ onb build_local(v3 n) {
 }
 
 // ------------------------------------------------------------------ rays
-struct RayPre {
+// What a ray's box tests read.
+struct RayBox {
     float ox, oy, oz;
     float ix, iy, iz; // 1 / dir (dir components below 2^-80 clamped)
-    float Sx, Sy, Sz;
     float tmin;
+};
+// A ray with what its triangle tests read as well.
+struct RayPre : RayBox {
+    float Sx, Sy, Sz;
     float okx, oky, okz; // origin permuted to (kx, ky, kz)
     int kx, ky, kz;
     float dx, dy, dz;
@@ -259,7 +263,7 @@ __device__ __forceinline__ void trav_init(Trav &T, const RayPre &r, float tmax, 
 
 // Visits one wide node: returns its {internal group, triangle group}.
 template <int W>
-__device__ __forceinline__ void visit_node(const uint4 *__restrict__ nodes, uint32_t child, const RayPre &r, uint32_t oct,
+__device__ __forceinline__ void visit_node(const uint4 *__restrict__ nodes, uint32_t child, const RayBox &r, uint32_t oct,
                                            float tfar, uint2 &ng, uint2 &tg) {
     using L = NodeLayout<W>;
     uint32_t w[L::WORDS];
@@ -414,66 +418,244 @@ __device__ __forceinline__ void traverse(const uint4 *__restrict__ nodes, const 
     occluded = T.occluded;
 }
 
-// Persistent traversal with per-lane ray refill (the "dynamic fetch" of Aila
-// & Laine, "Understanding the Efficiency of Ray Traversal on GPUs", HPG 2009).
-// A warp runs the loop with all lanes converged; a lane whose query is done
-// takes the next index from *head (one atomic per refill, for all idle lanes
-// at once) as soon as at least `min_refill` lanes are idle, so long queries
-// no longer hold the short ones' lanes idle.  Between refill checks each busy
-// lane advances its query by up to STEPS node visits.
+// ------------------------------------------------------------------ warp traversal
+// One ray per lane, the triangle tests shared by the warp.  A lane's node
+// visit leaves it zero to 24 pending triangles; tested by their own lanes they
+// keep the warp for the largest count of its lanes (9.1 of 32 lanes active per
+// instruction on the 1M-triangle soup).  Here the warp numbers all its pending
+// (ray, triangle) pairs by ballots, and its 32 lanes test 32 pairs at a time,
+// each lane any ray's triangle: the rays' triangle-test halves lie in the
+// warp's shared memory, which also takes them out of the registers.  A ray's
+// closest hit is the lexicographic minimum of (t, primitive) over its tests,
+// so who tests in what order does not change it.
+struct WarpRays {
+    float4 org[32];  // origin permuted to (kx, ky, kz); w = tmin
+    float4 shear[32]; // Sx, Sy, Sz; w = kx | ky << 2 | kz << 4 (bits)
+    uint2 pair[32];  // triangle slot, owning lane
+    uint2 res[32];   // t (bits) and primitive of the pair's hit; t = +inf when there is none
+    const float4 *tris[32]; // the ray's triangle array (rays of several scenes in one warp)
+};
+
+__device__ __forceinline__ void put_ray(WarpRays &sh, uint32_t lane, const RayPre &r, const float4 *tris) {
+    sh.org[lane] = make_float4(r.okx, r.oky, r.okz, r.tmin);
+    sh.shear[lane] = make_float4(r.Sx, r.Sy, r.Sz, __uint_as_float((uint32_t)(r.kx | r.ky << 2 | r.kz << 4)));
+    sh.tris[lane] = tris;
+}
+
+// The watertight test of triangle `slot` against the ray that `lane` stored.
+// False unless it crosses; a.w holds the primitive.
+__device__ __forceinline__ bool test_stored(const WarpRays &sh, uint32_t lane, uint32_t slot, const float4 *__restrict__ tris,
+                                            TriHit &h, uint32_t &prim, float &tmin) {
+    const float4 *tp = tris + (size_t)slot * 3;
+    const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
+    const float4 o = sh.org[lane], s = sh.shear[lane];
+    const uint32_t k = __float_as_uint(s.w);
+    RayPre r;
+    r.okx = o.x; r.oky = o.y; r.okz = o.z;
+    r.Sx = s.x; r.Sy = s.y; r.Sz = s.z;
+    r.kx = (int)(k & 3u); r.ky = (int)((k >> 2) & 3u); r.kz = (int)(k >> 4);
+    prim = __float_as_uint(a.w);
+    tmin = o.w;
+    return watertight(r, a, b, c, h);
+}
+
+// Traversal state of one lane's ray (its triangle-test half is in WarpRays).
+struct LaneTrav {
+    RayBox r;
+    uint2 ng; // {child_base, internal hits (traversal order) << 24 | imask}
+    uint2 tg; // {tri_base, pending triangle bits}
+    int sp;
+    float best_t;
+    uint32_t best_prim, best_slot;
+    uint32_t oct;
+    bool occluded;
+};
+
+__device__ __forceinline__ void lane_init(LaneTrav &T, const RayPre &r, float tmax, uint32_t root) {
+    T.r = r;
+    T.oct = (r.dx < 0.0f ? 4u : 0u) | (r.dy < 0.0f ? 2u : 0u) | (r.dz < 0.0f ? 1u : 0u);
+    T.ng = make_uint2(root, (1u << (24 + T.oct)) | 1u); // the root as child code 0 of a virtual parent
+    T.tg = make_uint2(0u, 0u);
+    T.sp = 0;
+    T.best_t = tmax;
+    T.best_prim = 0xFFFFFFFFu;
+    T.best_slot = 0xFFFFFFFFu;
+    T.occluded = false;
+}
+
+// Tests the pending triangles of the warp's lanes (all 32 lanes call it; a
+// lane without a ray has none).  When no lane has more than one, each lane
+// tests its own.
+template <bool ANY>
+__device__ __forceinline__ void warp_tris(LaneTrav &T, WarpRays &sh, const float4 *__restrict__ tris) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t cnt = (uint32_t)__popc(T.tg.y);
+    if (__ballot_sync(0xFFFFFFFFu, cnt != 0u) == 0u) return;
+    if (__ballot_sync(0xFFFFFFFFu, cnt > 1u) == 0u) {
+        if (cnt) {
+            const uint32_t slot = T.tg.x + (uint32_t)(__ffs(T.tg.y) - 1);
+            T.tg.y = 0u;
+            TriHit h;
+            uint32_t prim;
+            float tmin;
+            if (test_stored(sh, lane, slot, tris, h, prim, tmin)) {
+                if (ANY) {
+                    T.occluded = h.t > tmin && h.t < T.best_t;
+                } else if (accept_hit(h.t, prim, tmin, T.best_t, T.best_prim)) {
+                    T.best_t = h.t;
+                    T.best_prim = prim;
+                    T.best_slot = slot;
+                }
+            }
+        }
+        return;
+    }
+    // a pair's number: the counts of the lanes before, summed bit by bit
+    const uint32_t lt = (1u << lane) - 1u;
+    uint32_t next = 0u, total = 0u;
+#pragma unroll
+    for (int b = 0; b < 5; ++b) {
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, (cnt >> b) & 1u);
+        next += (uint32_t)__popc(m & lt) << b;
+        total += (uint32_t)__popc(m) << b;
+    }
+    for (uint32_t base = 0u; base < total; base += 32u) {
+        const uint32_t first = next;
+        while (T.tg.y != 0u && next < base + 32u) {
+            const uint32_t i = (uint32_t)(__ffs(T.tg.y) - 1);
+            T.tg.y &= T.tg.y - 1u;
+            sh.pair[next - base] = make_uint2(T.tg.x + i, lane);
+            ++next;
+        }
+        __syncwarp();
+        float t = INFINITY;
+        uint32_t prim = 0xFFFFFFFFu;
+        if (base + lane < total) {
+            const uint2 p = sh.pair[lane];
+            TriHit h;
+            float tmin;
+            if (test_stored(sh, p.y, p.x, sh.tris[p.y], h, prim, tmin) && h.t > tmin) t = h.t;
+        }
+        if (__ballot_sync(0xFFFFFFFFu, t < INFINITY)) {
+            sh.res[lane] = make_uint2(__float_as_uint(t), prim);
+            __syncwarp();
+            for (uint32_t k = first; k < next; ++k) {
+                const uint2 q = sh.res[k - base];
+                const float tk = __uint_as_float(q.x);
+                if (ANY) {
+                    if (tk < T.best_t) T.occluded = true;
+                } else if (tk < T.best_t || (tk == T.best_t && T.best_prim != 0xFFFFFFFFu && q.y < T.best_prim)) {
+                    T.best_t = tk;
+                    T.best_prim = q.y;
+                    T.best_slot = sh.pair[k - base].x;
+                }
+            }
+        }
+        __syncwarp(); // the pairs are read before the next window's are written
+    }
+}
+
+// Pops and visits one node of a lane's ray.
+template <int W>
+__device__ __forceinline__ void lane_visit(LaneTrav &T, uint2 *stack, const uint4 *__restrict__ nodes, uint32_t &err) {
+    if ((T.ng.y >> 24) == 0u) T.ng = stack[--T.sp];
+    const uint32_t pos = 31u - __clz(T.ng.y >> 24);
+    const uint32_t code = pos ^ T.oct;
+    T.ng.y &= ~(1u << (24 + pos));
+    const uint32_t child = T.ng.x + __popc(T.ng.y & ((1u << code) - 1u) & 0xFFu);
+    if ((T.ng.y >> 24) != 0u) {
+        if (T.sp < kStack) stack[T.sp++] = T.ng;
+        else err = 1u;
+    }
+    visit_node<W>(nodes, child, T.r, T.oct, T.best_t * kHitSlack, T.ng, T.tg);
+}
+
+// Traversal of a queue of rays by a warp, with per-lane refill (the "dynamic
+// fetch" of Aila & Laine, "Understanding the Efficiency of Ray Traversal on
+// GPUs", HPG 2009): a lane whose ray is done waits until `min_refill` lanes of
+// the warp do; they then hand over their results and take new rays together,
+// so that neither step runs for a single lane.
+//   take(cnt) -> first index of `cnt` queue entries (called by lane 0)
 //   fetch(idx, payload&, r&, tmax&, root&, nodes&, tris&) -> bool: loads query
 //        idx and its first traversal (BVH root node); false = the query was
 //        completed inside fetch (no traversal needed)
-//   advance(payload, const Trav&, r&, tmax&, root&) -> bool: called when a
+//   advance(payload, const LaneTrav&, r&, tmax&, root&) -> bool: called when a
 //        traversal ends; true = the query goes on with another traversal
 //        (the next placement of a scene), set up in r, tmax and root
-//   done(payload, const Trav&): consumes a finished query
-template <int W, bool ANY, bool COUNT, int STEPS, class Fetch, class Advance, class Done>
-__device__ __forceinline__ void dyn_traverse(unsigned int *head, unsigned int n, uint32_t min_refill, Fetch &&fetch,
+//   done(payload, const LaneTrav&): consumes a finished query (the lane's
+//        WarpRays entry still holds its ray)
+template <int W, bool ANY, bool COUNT, class Take, class Fetch, class Advance, class Done>
+__device__ __forceinline__ void dyn_traverse(WarpRays &sh, Take &&take, unsigned int n, uint32_t min_refill, Fetch &&fetch,
                                              Advance &&advance, Done &&done, TravStats &st, uint32_t &err) {
     const uint32_t lane = threadIdx.x & 31u;
-    bool has = false, exhausted = false;
+    enum { kEmpty, kRun, kEnded };
+    int state = kEmpty;
+    bool exhausted = false;
     uint32_t payload = 0;
-    RayPre r;
-    Trav T;
+    LaneTrav T;
+    T.tg = make_uint2(0u, 0u);
     uint2 stack[kStack];
     const uint4 *nodes = nullptr;
     const float4 *tris = nullptr;
     for (;;) {
-        const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !has);
-        if (!exhausted && idle != 0u && ((uint32_t)__popc(idle) >= min_refill || idle == 0xFFFFFFFFu)) {
-            const uint32_t cnt = (uint32_t)__popc(idle);
-            unsigned int base = 0;
-            if (lane == 0) base = atomicAdd(head, cnt);
-            base = __shfl_sync(0xFFFFFFFFu, base, 0);
-            if (base + cnt >= n) exhausted = true;
-            if (!has) {
-                const unsigned int my = base + (unsigned int)__popc(idle & ((1u << lane) - 1u));
-                if (my < n) {
-                    float tmax;
-                    uint32_t root = 0u;
-                    if (fetch(my, payload, r, tmax, root, nodes, tris)) {
-                        trav_init(T, r, tmax, root);
-                        has = true;
-                    }
-                }
-            }
-        }
-        if (!__any_sync(0xFFFFFFFFu, has)) {
-            if (exhausted) break;
-            continue;
-        }
-        if (has && trav_step<W, ANY, COUNT>(T, stack, nodes, tris, r, STEPS, st, err)) {
+        const uint32_t running = __ballot_sync(0xFFFFFFFFu, state == kRun);
+        const uint32_t waiting = exhausted ? __ballot_sync(0xFFFFFFFFu, state == kEnded) : ~running;
+        if (running == 0u || (uint32_t)__popc(waiting) >= min_refill) {
             float tmax;
             uint32_t root = 0u;
-            if (advance(payload, T, r, tmax, root)) {
-                trav_init(T, r, tmax, root);
-            } else {
-                has = false;
-                done(payload, T);
+            RayPre r;
+            bool start = false;
+            if (state == kEnded) {
+                if (advance(payload, T, r, tmax, root)) {
+                    start = true;
+                } else {
+                    done(payload, T);
+                    state = kEmpty;
+                }
+            }
+            const uint32_t idle = __ballot_sync(0xFFFFFFFFu, state == kEmpty);
+            if (!exhausted && idle != 0u) {
+                const uint32_t cnt = (uint32_t)__popc(idle);
+                unsigned int base = 0;
+                if (lane == 0) base = take(cnt);
+                base = __shfl_sync(0xFFFFFFFFu, base, 0);
+                if (base + cnt >= n) exhausted = true;
+                const unsigned int my = base + (unsigned int)__popc(idle & ((1u << lane) - 1u));
+                if (state == kEmpty && my < n) start = fetch(my, payload, r, tmax, root, nodes, tris);
+            }
+            if (start) {
+                lane_init(T, r, tmax, root);
+                put_ray(sh, lane, r, tris);
+                state = kRun;
+            }
+            __syncwarp();
+            if (!__any_sync(0xFFFFFFFFu, state == kRun)) {
+                if (exhausted) break;
+                continue;
             }
         }
+        if (state == kRun) {
+            lane_visit<W>(T, stack, nodes, err);
+            if (COUNT) {
+                st.nodes++;
+                st.tris += (uint32_t)__popc(T.tg.y);
+            }
+        }
+        warp_tris<ANY>(T, sh, tris);
+        if (state == kRun && (((T.ng.y >> 24) == 0u && T.sp == 0) || (ANY && T.occluded))) state = kEnded;
     }
+}
+
+// Barycentrics of a finished closest hit: the accepted test over again (a pure
+// function of ray and triangle), instead of three registers kept all the way.
+__device__ __forceinline__ void stored_uv(const WarpRays &sh, uint32_t lane, uint32_t slot, const float4 *__restrict__ tris,
+                                          float &u, float &v) {
+    TriHit h{0.0f, 0.0f, 0.0f, 1.0f};
+    uint32_t prim;
+    float tmin;
+    test_stored(sh, lane, slot, tris, h, prim, tmin);
+    u = h.V / h.det;
+    v = h.W / h.det;
 }
 
 } // namespace crg

@@ -1,10 +1,10 @@
 // traverse.cu — batched closest-hit / any-hit queries (the rtcIntersect1 /
 // rtcOccluded1 replacements, CRender src/objects/model.cpp:5-49).
 //
-// One thread per ray; rays are two 16-byte loads, hits one 16-byte store.
-// The wide nodes are read with 16-byte vector loads through the read-only
-// path; per-thread group stack of 64 entries (overflow raises the scene's
-// error word instead of trapping).
+// One ray per lane; rays are two 16-byte loads, hits one 16-byte store.  The
+// wide nodes are read with 16-byte vector loads through the read-only path;
+// per-lane group stack of 64 entries (overflow raises the scene's error word
+// instead of trapping).
 #include <algorithm>
 
 #include "render_common.cuh"
@@ -43,77 +43,68 @@ __global__ void __launch_bounds__(128) k_intersect_inst(rc::SceneDev S, const fl
     if (C.err) atomicOr(S.err, C.err);
 }
 
-// One thread per ray.  (A persistent-block variant that refilled idle lanes
-// from a shared-memory counter between traversal slices measured 21% slower
-// on the 1M-triangle soup: its extra state cost occupancy.)
+// One ray per lane, triangle tests shared by the warp, lanes refilled from the
+// block's run of `chunk` rays (dyn_traverse).  The run's counter lies in the
+// block's shared memory, so calls on several streams share nothing.  Bound by
+// instruction issue (75% of cycles) on incoherent rays; 8 blocks of 128 per SM
+// (64 registers).  1M-triangle soup, width 8: 16.8M closest hits 20.97 -> 14.97
+// ms against one thread per ray with its own triangle tests, 18.2 instead of
+// 9.1 lanes active; 5.0M any hits 2.73 -> 2.09 ms against per-lane refill
+// without shared tests.  9 and 10 blocks per SM (spills) were 2-3% slower.
 template <int W, bool ANY, bool COUNT>
 __global__ void __launch_bounds__(128, 8) k_intersect(const uint4 *__restrict__ nodes, const float4 *__restrict__ tris,
                                                    const float4 *__restrict__ rays, float4 *__restrict__ hits,
                                                    uint32_t *__restrict__ occluded, uint32_t *__restrict__ ncount,
-                                                   uint32_t *__restrict__ tcount, uint64_t n, uint32_t ntri,
-                                                   uint32_t *__restrict__ err) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float4 r0 = __ldg(&rays[2 * i]);
-    const float4 r1 = __ldg(&rays[2 * i + 1]);
-    float best_t = INFINITY, bu = 0.0f, bv = 0.0f;
-    uint32_t best_prim = 0xFFFFFFFFu, best_slot;
-    bool occ = false;
-    TravStats st{0, 0};
-    if (ntri > 0) {
-        const RayPre r = ray_prep(r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, r0.w);
-        uint32_t e = 0;
-        traverse<W, ANY, COUNT>(nodes, tris, r, r1.w, best_t, best_prim, best_slot, bu, bv, occ, st, e);
-        if (e) atomicOr(err, e);
-    }
-    if (ANY) {
-        occluded[i] = occ ? 1u : 0u;
-    } else {
-        if (best_prim == 0xFFFFFFFFu) {
-            best_t = INFINITY;
-            bu = bv = 0.0f;
-        }
-        hits[i] = make_float4(best_t, __uint_as_float(best_prim), bu, bv);
-    }
-    if (COUNT) {
-        if (ncount) ncount[i] = st.nodes;
-        if (tcount) tcount[i] = st.tris;
-    }
-}
-
-// Persistent variant with per-lane ray refill (dyn_traverse): a lane whose
-// ray is done takes the next ray index from *head while its warp's other
-// lanes are still traversing.
-template <int W, bool ANY>
-__global__ void __launch_bounds__(128) k_intersect_dyn(const uint4 *__restrict__ nodes, const float4 *__restrict__ tris,
-                                                     const float4 *__restrict__ rays, float4 *__restrict__ hits,
-                                                     uint32_t *__restrict__ occluded, unsigned int *head, uint32_t n,
-                                                     uint32_t refill, uint32_t *__restrict__ err) {
+                                                   uint32_t *__restrict__ tcount, uint64_t n, uint32_t chunk,
+                                                   uint32_t refill, uint32_t ntri, uint32_t *__restrict__ err) {
+    __shared__ WarpRays s_rays[4];
+    __shared__ unsigned int s_head;
+    if (threadIdx.x == 0) s_head = 0u;
+    __syncthreads();
+    WarpRays &sh = s_rays[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t first = (uint64_t)blockIdx.x * chunk;
+    const uint32_t count = (uint32_t)(n - first < chunk ? n - first : chunk);
     TravStats st{0, 0};
     uint32_t e = 0;
-    dyn_traverse<W, ANY, false, 4>(
-        head, n, refill,
-        [&](unsigned int i, uint32_t &payload, RayPre &r, float &tmax, uint32_t &root, const uint4 *&nd,
-            const float4 *&tr) {
+    auto put = [&](uint32_t i, float t, uint32_t prim, float u, float v) {
+        hits[first + i] = make_float4(t, __uint_as_float(prim), u, v);
+    };
+    auto put_counts = [&](uint32_t i) {
+        if (ncount) ncount[first + i] = st.nodes;
+        if (tcount) tcount[first + i] = st.tris;
+    };
+    dyn_traverse<W, ANY, COUNT>(
+        sh, [&](uint32_t cnt) { return atomicAdd(&s_head, cnt); }, count, refill,
+        [&](unsigned int i, uint32_t &payload, RayPre &r, float &tmax, uint32_t &, const uint4 *&nd, const float4 *&tr) {
+            if (COUNT) st = TravStats{0, 0};
+            if (ntri == 0) {
+                if (ANY) occluded[first + i] = 0u;
+                else put(i, INFINITY, 0xFFFFFFFFu, 0.0f, 0.0f);
+                if (COUNT) put_counts(i);
+                return false;
+            }
             payload = i;
-            root = 0u;
-            const float4 r0 = __ldg(&rays[2 * (size_t)i]);
-            const float4 r1 = __ldg(&rays[2 * (size_t)i + 1]);
+            const float4 r0 = __ldg(&rays[2 * (first + i)]);
+            const float4 r1 = __ldg(&rays[2 * (first + i) + 1]);
             r = ray_prep(r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, r0.w);
             tmax = r1.w;
             nd = nodes;
             tr = tris;
             return true;
         },
-        [](uint32_t, const Trav &, RayPre &, float &, uint32_t &) { return false; },
-        [&](uint32_t i, const Trav &T) {
+        [](uint32_t, const LaneTrav &, RayPre &, float &, uint32_t &) { return false; },
+        [&](uint32_t i, const LaneTrav &T) {
             if (ANY) {
-                occluded[i] = T.occluded ? 1u : 0u;
+                occluded[first + i] = T.occluded ? 1u : 0u;
             } else if (T.best_prim == 0xFFFFFFFFu) {
-                hits[i] = make_float4(INFINITY, __uint_as_float(0xFFFFFFFFu), 0.0f, 0.0f);
+                put(i, INFINITY, 0xFFFFFFFFu, 0.0f, 0.0f);
             } else {
-                hits[i] = make_float4(T.best_t, __uint_as_float(T.best_prim), T.best_V / T.best_det, T.best_W / T.best_det);
+                float u, v;
+                stored_uv(sh, lane, T.best_slot, tris, u, v);
+                put(i, T.best_t, T.best_prim, u, v);
             }
+            if (COUNT) put_counts(i);
         },
         st, e);
     if (e) atomicOr(err, e);
@@ -305,11 +296,12 @@ __global__ void __launch_bounds__(128) k_intersect_warp(const uint4 *__restrict_
     if (e) atomicOr(err, e);
 }
 
-// Any-hit queries use the refill kernel (threshold 4 idle lanes): on the
-// 1M-triangle soup with 16M shadow rays it measured 1862 against 1364 Mrays/s
-// for one thread per ray.  Closest-hit queries stay one thread per ray (813
-// against 781 Mrays/s).
-constexpr uint32_t kAnyRefill = 4;
+// Idle lanes that make a warp refill: 4 / 8 / 12 measured 15.13 / 15.04 / 15.43
+// ms on the soup's 16.8M closest hits, 2.12 / 2.10 / 2.15 ms on 5.0M any hits.
+constexpr uint32_t kRefill = 8;
+// Rays of a block at most: 1024 / 2048 / 8192 measured 14.97 / 15.04 / 15.91 ms
+// (closest) and 2.28 / 2.10 / 2.12 ms (any).
+constexpr uint32_t kChunkMax = 2048;
 
 template <int W>
 void launch_warp(const crg_scene *s, const crg_ray *rays, crg_hit *hits, uint32_t *occluded, uint64_t n, bool any,
@@ -342,38 +334,24 @@ void launch_w(const crg_scene *s, const crg_ray *rays, crg_hit *hits, uint32_t *
         if (tris) cudaMemsetAsync(tris, 0, 4 * n, st);
         return;
     }
-    if (any && n >= (1u << 16) && n < 0xFFFF0000ull && s->ntri > 0) {
-        int per_sm = 0;
-        if (any) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_intersect_dyn<W, true>, 128, 0);
-        else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_intersect_dyn<W, false>, 128, 0);
-        const uint32_t grid = (uint32_t)(std::max(s->ctx->sm_count, 1) * std::max(per_sm, 1));
-        unsigned int *head = (unsigned int *)s->qhead.ptr;
-        cudaMemsetAsync(head, 0, sizeof(unsigned int), st);
-        const uint4 *nd = (const uint4 *)s->wide.ptr;
-        const float4 *tr = (const float4 *)s->tris.ptr;
-        if (any)
-            k_intersect_dyn<W, true><<<grid, 128, 0, st>>>(nd, tr, (const float4 *)rays, nullptr, occluded, head,
-                                                           (uint32_t)n, kAnyRefill, (uint32_t *)s->err.ptr);
-        else
-            k_intersect_dyn<W, false><<<grid, 128, 0, st>>>(nd, tr, (const float4 *)rays, (float4 *)hits, nullptr, head,
-                                                            (uint32_t)n, kAnyRefill, (uint32_t *)s->err.ptr);
-        return;
-    }
-    const uint32_t T = 128;
-    const uint64_t blocks = (n + T - 1) / T;
+    // a block's run of rays: long enough that its warps mostly run full, short
+    // enough that every SM gets several blocks one after the other
+    const uint64_t resident = (uint64_t)std::max(s->ctx->sm_count, 1) * 8;
+    const uint64_t share = (n / (resident * 6) + 127) / 128 * 128;
+    const uint32_t chunk = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(share, 128), kChunkMax);
+    const uint64_t blocks = (n + chunk - 1) / chunk;
     const uint4 *nd = (const uint4 *)s->wide.ptr;
     const float4 *tr = (const float4 *)s->tris.ptr;
     uint32_t *err = (uint32_t *)s->err.ptr;
-    const bool count = nodes || tris;
     if (any)
-        k_intersect<W, true, false><<<blocks, T, 0, st>>>(nd, tr, (const float4 *)rays, nullptr, occluded, nullptr, nullptr, n,
-                                                           s->ntri, err);
-    else if (count)
-        k_intersect<W, false, true><<<blocks, T, 0, st>>>(nd, tr, (const float4 *)rays, (float4 *)hits, nullptr, nodes, tris, n,
-                                                           s->ntri, err);
+        k_intersect<W, true, false><<<blocks, 128, 0, st>>>(nd, tr, (const float4 *)rays, nullptr, occluded, nullptr, nullptr,
+                                                           n, chunk, kRefill, s->ntri, err);
+    else if (nodes || tris)
+        k_intersect<W, false, true><<<blocks, 128, 0, st>>>(nd, tr, (const float4 *)rays, (float4 *)hits, nullptr, nodes, tris,
+                                                           n, chunk, kRefill, s->ntri, err);
     else
-        k_intersect<W, false, false><<<blocks, T, 0, st>>>(nd, tr, (const float4 *)rays, (float4 *)hits, nullptr, nullptr,
-                                                            nullptr, n, s->ntri, err);
+        k_intersect<W, false, false><<<blocks, 128, 0, st>>>(nd, tr, (const float4 *)rays, (float4 *)hits, nullptr, nullptr,
+                                                            nullptr, n, chunk, kRefill, s->ntri, err);
 }
 
 } // namespace
