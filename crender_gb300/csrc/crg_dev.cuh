@@ -173,14 +173,16 @@ __device__ __forceinline__ bool watertight(const RayPre &r, float4 a, float4 b, 
     float U = Cx * By - Cy * Bx;
     float V = Ax * Cy - Ay * Cx;
     float W = Bx * Ay - By * Ax;
-    if (U == 0.0f || V == 0.0f || W == 0.0f) {
+    // least / greatest of three (one instruction each; NaN operands are passed over, as the
+    // comparisons one by one do)
+    if (fminf(fminf(fabsf(U), fabsf(V)), fabsf(W)) == 0.0f) {
         U = (float)((double)Cx * (double)By - (double)Cy * (double)Bx);
         V = (float)((double)Ax * (double)Cy - (double)Ay * (double)Cx);
         W = (float)((double)Bx * (double)Ay - (double)By * (double)Ax);
     }
-    if ((U < 0.0f || V < 0.0f || W < 0.0f) && (U > 0.0f || V > 0.0f || W > 0.0f)) return false;
-    const float det = (U + V) + W;
-    if (det == 0.0f) return false;
+    float det = (U + V) + W;
+    const bool cross = !(fminf(fminf(U, V), W) < 0.0f && fmaxf(fmaxf(U, V), W) > 0.0f) && det != 0.0f;
+    det = cross ? det : 1.0f;
     const float Az = r.Sz * Akz;
     const float Bz = r.Sz * Bkz;
     const float Cz = r.Sz * Ckz;
@@ -189,7 +191,7 @@ __device__ __forceinline__ bool watertight(const RayPre &r, float4 a, float4 b, 
     h.V = V;
     h.W = W;
     h.det = det;
-    return true;
+    return cross;
 }
 
 __device__ __forceinline__ bool accept_hit(float t, uint32_t prim, float tmin, float best_t, uint32_t best_prim) {
@@ -213,11 +215,18 @@ template <int W> __device__ __forceinline__ uint32_t nbyte(const uint32_t *w, in
     return (w[b >> 2] >> ((b & 3) * 8)) & 0xFFu;
 }
 
-// Byte k of `word` as an exact float: 2^23 + q assembled by PRMT, minus 2^23.
-__device__ __forceinline__ float2 qpair(uint32_t word, int k) {
-    const float2 biased = make_float2(__uint_as_float(__byte_perm(word, 0x4B000000u, 0x7440u | k)),
-                                      __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7440u | (k + 1))));
-    return __fadd2_rn(biased, make_float2(-8388608.0f, -8388608.0f));
+// Bytes k and k + 1 of `word` as exact floats 2^15 + q: one PRMT each (q is the
+// second byte of the float's bits).
+__device__ __forceinline__ float2 qbias(uint32_t word, int k) {
+    return make_float2(__uint_as_float(__byte_perm(word, 0x47000000u, 0x7604u | (uint32_t)k << 4)),
+                       __uint_as_float(__byte_perm(word, 0x47000000u, 0x7604u | (uint32_t)(k + 1) << 4)));
+}
+
+// Every byte of x filled with its top bit.
+__device__ __forceinline__ uint32_t byte_sign(uint32_t x) {
+    uint32_t r;
+    asm("prmt.b32 %0, %1, 0, 0xBA98;" : "=r"(r) : "r"(x));
+    return r;
 }
 
 struct TravStats {
@@ -292,26 +301,39 @@ __device__ __forceinline__ void visit_node(const uint4 *__restrict__ nodes, uint
         constexpr int LO = (24 + W) / 4, HI = (24 + 4 * W) / 4, ME = 24 / 4;
         const bool nxs = r.ix < 0.0f, nys = r.iy < 0.0f, nzs = r.iz < 0.0f;
         const float2 sx2 = make_float2(sx, sx), sy2 = make_float2(sy, sy), sz2 = make_float2(sz, sz);
-        const float2 ox2 = make_float2(ox, ox), oy2 = make_float2(oy, oy), oz2 = make_float2(oz, oz);
+        // the plane parameters are formed from 2^15 + q, so the offset takes 2^15 quanta off:
+        // that rounds to within 2^-9 quantum, and the boxes hold a whole quantum of slack per side
+        const float bx = __fmaf_rn(-32768.0f, sx, ox), by = __fmaf_rn(-32768.0f, sy, oy), bz = __fmaf_rn(-32768.0f, sz, oz);
+        const float2 ox2 = make_float2(bx, bx), oy2 = make_float2(by, by), oz2 = make_float2(bz, bz);
+        const uint32_t oct4 = oct * 0x01010101u;
 #pragma unroll
-        for (int p = 0; p < W / 2; ++p) {
-            const int wi = (2 * p) >> 2, bo = (2 * p) & 3;
+        for (int wi = 0; wi < QW; ++wi) {
             const uint32_t lx = w[LO + 0 * QW + wi], hx = w[HI + 0 * QW + wi];
             const uint32_t ly = w[LO + 1 * QW + wi], hy = w[HI + 1 * QW + wi];
             const uint32_t lz = w[LO + 2 * QW + wi], hz = w[HI + 2 * QW + wi];
-            const float2 txn = __ffma2_rn(qpair(nxs ? hx : lx, bo), sx2, ox2);
-            const float2 txf = __ffma2_rn(qpair(nxs ? lx : hx, bo), sx2, ox2);
-            const float2 tyn = __ffma2_rn(qpair(nys ? hy : ly, bo), sy2, oy2);
-            const float2 tyf = __ffma2_rn(qpair(nys ? ly : hy, bo), sy2, oy2);
-            const float2 tzn = __ffma2_rn(qpair(nzs ? hz : lz, bo), sz2, oz2);
-            const float2 tzf = __ffma2_rn(qpair(nzs ? lz : hz, bo), sz2, oz2);
+            const uint32_t xn = nxs ? hx : lx, xf = nxs ? lx : hx;
+            const uint32_t yn = nys ? hy : ly, yf = nys ? ly : hy;
+            const uint32_t zn = nzs ? hz : lz, zf = nzs ? lz : hz;
+            // four slots' bit values and positions at once: an internal child (meta 24..31 with bits
+            // 3 and 4 set) takes bit 24 + (code ^ oct), a leaf the bits of its triangles
             const uint32_t mw = w[ME + wi];
+            const uint32_t inner = mw & (mw << 1) & 0x10101010u;
+            const uint32_t pos4 = mw ^ (byte_sign(inner << 3) & oct4);
+            const uint32_t val4 = (mw >> 5) & 0x07070707u;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const float tn = fmaxf(fmaxf(h ? txn.y : txn.x, h ? tyn.y : tyn.x), fmaxf(h ? tzn.y : tzn.x, r.tmin));
-                const float tf = fminf(fminf(h ? txf.y : txf.x, h ? tyf.y : tyf.x), fminf(h ? tzf.y : tzf.x, tfar));
-                const uint32_t meta = (mw >> (8 * (bo + h))) & 0xFFu;
-                if (tn <= tf * 1.00000095f) bits |= (meta >> 5) << (meta & 31u);
+            for (int bo = 0; bo < 4; bo += 2) {
+                const float2 txn = __ffma2_rn(qbias(xn, bo), sx2, ox2), txf = __ffma2_rn(qbias(xf, bo), sx2, ox2);
+                const float2 tyn = __ffma2_rn(qbias(yn, bo), sy2, oy2), tyf = __ffma2_rn(qbias(yf, bo), sy2, oy2);
+                const float2 tzn = __ffma2_rn(qbias(zn, bo), sz2, oz2), tzf = __ffma2_rn(qbias(zf, bo), sz2, oz2);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float tn = fmaxf(fmaxf(h ? txn.y : txn.x, h ? tyn.y : tyn.x), fmaxf(h ? tzn.y : tzn.x, r.tmin));
+                    const float tf = fminf(fminf(h ? txf.y : txf.x, h ? tyf.y : tyf.x), fminf(h ? tzf.y : tzf.x, tfar));
+                    const int k = bo + h;
+                    // the shift takes its count modulo 32: the position's low five bits
+                    const uint32_t v = __funnelshift_l(0u, __byte_perm(val4, 0u, 0x4440u | (uint32_t)k), pos4 >> (8 * k));
+                    if (tn <= tf * 1.00000095f) bits |= v;
+                }
             }
         }
     } else {
@@ -332,15 +354,12 @@ __device__ __forceinline__ void visit_node(const uint4 *__restrict__ nodes, uint
             const float tz1 = __fmaf_rn(r.iz >= 0.0f ? qhz : qlz, sz, oz);
             const float tn = fmaxf(fmaxf(tx0, ty0), fmaxf(tz0, r.tmin));
             const float tf = fminf(fminf(tx1, ty1), fminf(tz1, tfar));
-            if (tn <= tf * 1.00000095f) bits |= (meta >> 5) << (meta & 31u);
+            const uint32_t inner = (meta >> 3) & (meta >> 4) & 1u;
+            if (tn <= tf * 1.00000095f) bits |= (meta >> 5) << ((meta ^ (inner ? oct : 0u)) & 31u);
         }
     }
-    // internal hits by octant code -> traversal order (bit position code ^ oct)
-    uint32_t m = bits >> 24;
-    if (oct & 1u) m = ((m & 0x55u) << 1) | ((m >> 1) & 0x55u);
-    if (oct & 2u) m = ((m & 0x33u) << 2) | ((m >> 2) & 0x33u);
-    if (oct & 4u) m = ((m & 0x0Fu) << 4) | ((m >> 4) & 0x0Fu);
-    ng = make_uint2(w[4], (m << 24) | imask);
+    // internal hits lie in traversal order (bit position code ^ oct)
+    ng = make_uint2(w[4], (bits & 0xFF000000u) | imask);
     tg = make_uint2(w[5], bits & 0x00FFFFFFu);
 }
 
@@ -427,12 +446,20 @@ __device__ __forceinline__ void traverse(const uint4 *__restrict__ nodes, const 
 // each lane any ray's triangle: the rays' triangle-test halves lie in the
 // warp's shared memory, which also takes them out of the registers.  A ray's
 // closest hit is the lexicographic minimum of (t, primitive) over its tests,
-// so who tests in what order does not change it.
+// so who tests in what order does not change it.  The kernels are bound by
+// instruction issue, so what counts is instructions per visit: a lane finds its
+// pair from one OR-reduction and two shared loads (owners writing their pairs in
+// a loop: 14.6 against 13.6 ms on the soup's 16.8M closest hits), owners read
+// only their hits, and the test and the stack push run without branches
+// (13.25 ms).  A separate path for warps without a lane of several pairs cost
+// more than it saved (13.25 against 12.78 ms).
 struct WarpRays {
-    float4 org[32];  // origin permuted to (kx, ky, kz); w = tmin
+    float4 org[32];   // origin permuted to (kx, ky, kz); w = tmin
     float4 shear[32]; // Sx, Sy, Sz; w = kx | ky << 2 | kz << 4 (bits)
-    uint2 pair[32];  // triangle slot, owning lane
-    uint2 res[32];   // t (bits) and primitive of the pair's hit; t = +inf when there is none
+    uint4 group[32];  // a lane's pending triangles: tri_base, bits, number of its first pair
+    uint2 res[32];    // t (bits) and primitive of the hit of the window's pair k
+    uint32_t slot[32]; // the pair's triangle slot
+    uint32_t owner[32]; // lane whose pairs start at window position k
     const float4 *tris[32]; // the ray's triangle array (rays of several scenes in one warp)
 };
 
@@ -484,93 +511,100 @@ __device__ __forceinline__ void lane_init(LaneTrav &T, const RayPre &r, float tm
 }
 
 // Tests the pending triangles of the warp's lanes (all 32 lanes call it; a
-// lane without a ray has none).  When no lane has more than one, each lane
-// tests its own.
+// lane without a ray has none), in windows of 32 pairs.
 template <bool ANY>
 __device__ __forceinline__ void warp_tris(LaneTrav &T, WarpRays &sh, const float4 *__restrict__ tris) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t cnt = (uint32_t)__popc(T.tg.y);
     if (__ballot_sync(0xFFFFFFFFu, cnt != 0u) == 0u) return;
-    if (__ballot_sync(0xFFFFFFFFu, cnt > 1u) == 0u) {
-        if (cnt) {
-            const uint32_t slot = T.tg.x + (uint32_t)(__ffs(T.tg.y) - 1);
-            T.tg.y = 0u;
+    // a pair's number: the counts of the lanes before, summed bit by bit
+    const uint32_t lt = (1u << lane) - 1u;
+    uint32_t first = 0u, total = 0u;
+    const uint32_t m0 = __ballot_sync(0xFFFFFFFFu, cnt & 1u), m1 = __ballot_sync(0xFFFFFFFFu, cnt & 2u);
+    first = (uint32_t)__popc(m0 & lt) + 2u * (uint32_t)__popc(m1 & lt);
+    total = (uint32_t)__popc(m0) + 2u * (uint32_t)__popc(m1);
+    if (__ballot_sync(0xFFFFFFFFu, cnt > 3u)) {
+#pragma unroll
+        for (int b = 2; b < 5; ++b) {
+            const uint32_t m = __ballot_sync(0xFFFFFFFFu, (cnt >> b) & 1u);
+            first += (uint32_t)__popc(m & lt) << b;
+            total += (uint32_t)__popc(m) << b;
+        }
+    }
+    if (cnt) sh.group[lane] = make_uint4(T.tg.x, T.tg.y, first, 0u);
+    T.tg.y = 0u;
+    for (uint32_t base = 0u; base < total; base += 32u) {
+        // the lane's pairs in this window: positions [at, at + mine)
+        const uint32_t lo = max(first, base), hi = min(first + cnt, base + 32u);
+        const bool has = lo < hi;
+        const uint32_t at = lo - base;
+        if (has) sh.owner[at] = lane;
+        const uint32_t starts = __reduce_or_sync(0xFFFFFFFFu, has ? 1u << at : 0u);
+        __syncwarp();
+        float t = INFINITY;
+        if (base + lane < total) {
+            const uint32_t own = sh.owner[31 - __clz(starts & ((2u << lane) - 1u))];
+            const uint4 g = sh.group[own];
+            uint32_t bits = g.y;
+            uint32_t rank = base + lane - g.z;
+            if (rank >= 1u) bits &= bits - 1u;
+            if (rank >= 2u) bits &= bits - 1u;
+            while (rank >= 3u) {
+                bits &= bits - 1u;
+                --rank;
+            }
+            const uint32_t slot = g.x + (uint32_t)(__ffs(bits) - 1);
             TriHit h;
             uint32_t prim;
             float tmin;
-            if (test_stored(sh, lane, slot, tris, h, prim, tmin)) {
-                if (ANY) {
-                    T.occluded = h.t > tmin && h.t < T.best_t;
-                } else if (accept_hit(h.t, prim, tmin, T.best_t, T.best_prim)) {
-                    T.best_t = h.t;
-                    T.best_prim = prim;
-                    T.best_slot = slot;
-                }
+            if (test_stored(sh, own, slot, sh.tris[own], h, prim, tmin) && h.t > tmin) {
+                t = h.t;
+                sh.res[lane] = make_uint2(__float_as_uint(t), prim);
+                sh.slot[lane] = slot;
             }
         }
-        return;
-    }
-    // a pair's number: the counts of the lanes before, summed bit by bit
-    const uint32_t lt = (1u << lane) - 1u;
-    uint32_t next = 0u, total = 0u;
-#pragma unroll
-    for (int b = 0; b < 5; ++b) {
-        const uint32_t m = __ballot_sync(0xFFFFFFFFu, (cnt >> b) & 1u);
-        next += (uint32_t)__popc(m & lt) << b;
-        total += (uint32_t)__popc(m) << b;
-    }
-    for (uint32_t base = 0u; base < total; base += 32u) {
-        const uint32_t first = next;
-        while (T.tg.y != 0u && next < base + 32u) {
-            const uint32_t i = (uint32_t)(__ffs(T.tg.y) - 1);
-            T.tg.y &= T.tg.y - 1u;
-            sh.pair[next - base] = make_uint2(T.tg.x + i, lane);
-            ++next;
-        }
+        const uint32_t hits = __ballot_sync(0xFFFFFFFFu, t < INFINITY);
         __syncwarp();
-        float t = INFINITY;
-        uint32_t prim = 0xFFFFFFFFu;
-        if (base + lane < total) {
-            const uint2 p = sh.pair[lane];
-            TriHit h;
-            float tmin;
-            if (test_stored(sh, p.y, p.x, sh.tris[p.y], h, prim, tmin) && h.t > tmin) t = h.t;
-        }
-        if (__ballot_sync(0xFFFFFFFFu, t < INFINITY)) {
-            sh.res[lane] = make_uint2(__float_as_uint(t), prim);
-            __syncwarp();
-            for (uint32_t k = first; k < next; ++k) {
-                const uint2 q = sh.res[k - base];
-                const float tk = __uint_as_float(q.x);
-                if (ANY) {
-                    if (tk < T.best_t) T.occluded = true;
-                } else if (tk < T.best_t || (tk == T.best_t && T.best_prim != 0xFFFFFFFFu && q.y < T.best_prim)) {
-                    T.best_t = tk;
-                    T.best_prim = q.y;
-                    T.best_slot = sh.pair[k - base].x;
-                }
+        // the lane's own hits (2u << 31 wraps to 0: all positions from `at` on)
+        uint32_t own_hits = has ? hits & ((2u << (hi - base - 1u)) - 1u) & ~((1u << at) - 1u) : 0u;
+        while (own_hits) {
+            const uint32_t k = (uint32_t)(__ffs(own_hits) - 1);
+            own_hits &= own_hits - 1u;
+            const uint2 q = sh.res[k];
+            const float tk = __uint_as_float(q.x);
+            if (ANY) {
+                if (tk < T.best_t) T.occluded = true;
+            } else if (tk < T.best_t || (tk == T.best_t && T.best_prim != 0xFFFFFFFFu && q.y < T.best_prim)) {
+                T.best_t = tk;
+                T.best_prim = q.y;
+                T.best_slot = sh.slot[k];
             }
         }
-        __syncwarp(); // the pairs are read before the next window's are written
+        __syncwarp(); // the window is read before the next one overwrites it
     }
 }
 
-// Pops and visits one node of a lane's ray.
+// Visits the next node of a lane's ray; afterwards ng holds the group to go on
+// with (none left: the ray has no nodes to visit any more).
 template <int W>
 __device__ __forceinline__ void lane_visit(LaneTrav &T, uint2 *stack, const uint4 *__restrict__ nodes, uint32_t &err) {
-    if ((T.ng.y >> 24) == 0u) T.ng = stack[--T.sp];
-    const uint32_t pos = 31u - __clz(T.ng.y >> 24);
-    const uint32_t code = pos ^ T.oct;
-    T.ng.y &= ~(1u << (24 + pos));
-    const uint32_t child = T.ng.x + __popc(T.ng.y & ((1u << code) - 1u) & 0xFFu);
-    if ((T.ng.y >> 24) != 0u) {
-        if (T.sp < kStack) stack[T.sp++] = T.ng;
-        else err = 1u;
-    }
+    const uint32_t top = 31u - __clz(T.ng.y); // 24 + (code ^ oct)
+    const uint32_t code = (top - 24u) ^ T.oct;
+    T.ng.y &= ~(1u << top);
+    const uint32_t child = T.ng.x + __popc(T.ng.y & ((1u << code) - 1u));
+    const bool more = T.ng.y >= 1u << 24, fits = T.sp < kStack;
+    if (more && fits) stack[T.sp] = T.ng;
+    err |= more && !fits ? 1u : 0u;
+    T.sp += more && fits ? 1 : 0;
     visit_node<W>(nodes, child, T.r, T.oct, T.best_t * kHitSlack, T.ng, T.tg);
+    if (T.ng.y < 1u << 24 && T.sp > 0) T.ng = stack[--T.sp];
 }
 
-// Traversal of a queue of rays by a warp, with per-lane refill (the "dynamic
+// Traversal of a queue of rays by a warp: node visits for as long as at least
+// VISITORS lanes have no triangles pending, then the pending triangles of all
+// lanes; one visit yields 0.55 triangles per ray on the soup, so a second visit
+// by the lanes that got none nearly fills the 32 test places (every ray still
+// tests a visit's triangles before its next visit).  With per-lane refill (the "dynamic
 // fetch" of Aila & Laine, "Understanding the Efficiency of Ray Traversal on
 // GPUs", HPG 2009): a lane whose ray is done waits until `min_refill` lanes of
 // the warp do; they then hand over their results and take new rays together,
@@ -584,7 +618,7 @@ __device__ __forceinline__ void lane_visit(LaneTrav &T, uint2 *stack, const uint
 //        (the next placement of a scene), set up in r, tmax and root
 //   done(payload, const LaneTrav&): consumes a finished query (the lane's
 //        WarpRays entry still holds its ray)
-template <int W, bool ANY, bool COUNT, class Take, class Fetch, class Advance, class Done>
+template <int W, bool ANY, bool COUNT, uint32_t VISITORS, class Take, class Fetch, class Advance, class Done>
 __device__ __forceinline__ void dyn_traverse(WarpRays &sh, Take &&take, unsigned int n, uint32_t min_refill, Fetch &&fetch,
                                              Advance &&advance, Done &&done, TravStats &st, uint32_t &err) {
     const uint32_t lane = threadIdx.x & 31u;
@@ -593,7 +627,8 @@ __device__ __forceinline__ void dyn_traverse(WarpRays &sh, Take &&take, unsigned
     bool exhausted = false;
     uint32_t payload = 0;
     LaneTrav T;
-    T.tg = make_uint2(0u, 0u);
+    T.ng = T.tg = make_uint2(0u, 0u);
+    T.occluded = false;
     uint2 stack[kStack];
     const uint4 *nodes = nullptr;
     const float4 *tris = nullptr;
@@ -634,15 +669,21 @@ __device__ __forceinline__ void dyn_traverse(WarpRays &sh, Take &&take, unsigned
                 continue;
             }
         }
-        if (state == kRun) {
-            lane_visit<W>(T, stack, nodes, err);
-            if (COUNT) {
-                st.nodes++;
-                st.tris += (uint32_t)__popc(T.tg.y);
+        for (;;) {
+            const bool can = T.tg.y == 0u && T.ng.y >= 1u << 24;
+            const uint32_t visitors = __ballot_sync(0xFFFFFFFFu, can);
+            if (visitors == 0u || ((uint32_t)__popc(visitors) < VISITORS && __any_sync(0xFFFFFFFFu, T.tg.y != 0u))) break;
+            if (can) {
+                lane_visit<W>(T, stack, nodes, err);
+                if (COUNT) {
+                    st.nodes++;
+                    st.tris += (uint32_t)__popc(T.tg.y);
+                }
             }
         }
         warp_tris<ANY>(T, sh, tris);
-        if (state == kRun && (((T.ng.y >> 24) == 0u && T.sp == 0) || (ANY && T.occluded))) state = kEnded;
+        if (ANY && T.occluded) T.ng.y = 0u;
+        if (state == kRun && T.ng.y < 1u << 24) state = kEnded;
     }
 }
 

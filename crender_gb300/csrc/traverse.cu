@@ -43,14 +43,19 @@ __global__ void __launch_bounds__(128) k_intersect_inst(rc::SceneDev S, const fl
     if (C.err) atomicOr(S.err, C.err);
 }
 
+// Lanes without pending triangles below which a warp turns to the triangle
+// tests: 16 / 20 / 24 measured 12.15 / 11.91 / 12.22 ms on the soup's 16.8M
+// closest hits, 1.76 / 1.76 / 1.79 ms on 5.0M any hits.
+constexpr uint32_t kVisitors = 20;
+
 // One ray per lane, triangle tests shared by the warp, lanes refilled from the
 // block's run of `chunk` rays (dyn_traverse).  The run's counter lies in the
 // block's shared memory, so calls on several streams share nothing.  Bound by
 // instruction issue (75% of cycles) on incoherent rays; 8 blocks of 128 per SM
-// (64 registers).  1M-triangle soup, width 8: 16.8M closest hits 20.97 -> 14.97
-// ms against one thread per ray with its own triangle tests, 18.2 instead of
-// 9.1 lanes active; 5.0M any hits 2.73 -> 2.09 ms against per-lane refill
-// without shared tests.  9 and 10 blocks per SM (spills) were 2-3% slower.
+// (64 registers).  1M-triangle soup, width 8: 16.8M closest hits 20.97 -> 11.91
+// ms against one thread per ray with its own triangle tests (9.1 lanes active),
+// 5.0M any hits 2.73 -> 1.76 ms against per-lane refill without shared tests.
+// 9 and 10 blocks per SM (spills) were 2-3% slower.
 template <int W, bool ANY, bool COUNT>
 __global__ void __launch_bounds__(128, 8) k_intersect(const uint4 *__restrict__ nodes, const float4 *__restrict__ tris,
                                                    const float4 *__restrict__ rays, float4 *__restrict__ hits,
@@ -74,7 +79,7 @@ __global__ void __launch_bounds__(128, 8) k_intersect(const uint4 *__restrict__ 
         if (ncount) ncount[first + i] = st.nodes;
         if (tcount) tcount[first + i] = st.tris;
     };
-    dyn_traverse<W, ANY, COUNT>(
+    dyn_traverse<W, ANY, COUNT, kVisitors>(
         sh, [&](uint32_t cnt) { return atomicAdd(&s_head, cnt); }, count, refill,
         [&](unsigned int i, uint32_t &payload, RayPre &r, float &tmax, uint32_t &, const uint4 *&nd, const float4 *&tr) {
             if (COUNT) st = TravStats{0, 0};

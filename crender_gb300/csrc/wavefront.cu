@@ -404,9 +404,16 @@ __global__ void __launch_bounds__(256) k_wf_shadow(Wf w) {
     }
 }
 
+// Lanes without pending triangles below which a warp of the traversal stages
+// turns to the triangle tests: 33 (every visit) / 20 / 16 rendered the ten-view
+// batch in 314 / 301 / 298 ms.
+constexpr uint32_t kVisitors = 16;
+
 // Extend with per-lane ray refill and triangle tests shared by the warp
 // (dyn_traverse): the same hits as k_wf_extend.  With the shared tests a batch
-// of ten views (388M samples) takes 308 instead of 317 ms.
+// of ten views (388M samples) takes 308 instead of 317 ms.  4 blocks of 256 per
+// SM (64 registers): extend 111 ms of that batch, against 114 at 5 blocks (48
+// registers, spills) and 115 at 3.
 // PL: the scenes' placements.  0: none (one mesh per scene).  1: at most
 // kLoopPlacements per scene, traced one after the other as
 // closest_placement_loop does.  2: placements through the top-level tree, as
@@ -416,7 +423,7 @@ __global__ void __launch_bounds__(256) k_wf_shadow(Wf w) {
 // ray that reaches no placement box runs one empty traversal (tmax below
 // tmin) so that every query passes through done.
 template <int W, bool CNT, int PL>
-__global__ void __launch_bounds__(256, 5) k_wf_extend_dyn(Wf w) {
+__global__ void __launch_bounds__(256, 4) k_wf_extend_dyn(Wf w) {
     Ctrl *c = w.ctrl;
     const unsigned int n = c->in_count;
     const uint32_t *in = q_in(w, *c);
@@ -438,7 +445,7 @@ __global__ void __launch_bounds__(256, 5) k_wf_extend_dyn(Wf w) {
         root = __ldg(&Sp->inst_root[k]);
     };
     extern __shared__ WarpRays s_rays[];
-    dyn_traverse<W, false, CNT>(
+    dyn_traverse<W, false, CNT, kVisitors>(
         s_rays[threadIdx.x >> 5], [&](uint32_t cnt) { return atomicAdd(&c->head_ext, cnt); }, n, w.refill,
         [&](unsigned int qi, uint32_t &slot, RayPre &r, float &tmax, uint32_t &root, const uint4 *&nodes,
             const float4 *&tris) {
@@ -524,7 +531,7 @@ __global__ void __launch_bounds__(256, 5) k_wf_extend_dyn(Wf w) {
 // (occluded_placement_loop, occluded_placements), stopping at the first
 // placement that occludes.
 template <int W, bool CNT, int PL>
-__global__ void __launch_bounds__(256, 5) k_wf_shadow_dyn(Wf w) {
+__global__ void __launch_bounds__(256, 4) k_wf_shadow_dyn(Wf w) {
     Ctrl *c = w.ctrl;
     const unsigned int n = c->sh_count;
     TravStats st{0, 0};
@@ -544,7 +551,7 @@ __global__ void __launch_bounds__(256, 5) k_wf_shadow_dyn(Wf w) {
         root = __ldg(&Sp->inst_root[k]);
     };
     extern __shared__ WarpRays s_rays[];
-    dyn_traverse<W, true, CNT>(
+    dyn_traverse<W, true, CNT, kVisitors>(
         s_rays[threadIdx.x >> 5], [&](uint32_t cnt) { return atomicAdd(&c->head_sh, cnt); }, n, w.refill_sh,
         [&](unsigned int qi, uint32_t &slot, RayPre &r, float &tmax, uint32_t &root, const uint4 *&nodes,
             const float4 *&tris) {
