@@ -546,6 +546,8 @@ __global__ void __launch_bounds__(128) k_treelet(Tree T, uint32_t n, uint32_t *_
 struct Collapse {
     Tree T;
     const float *verts;  // the BVH's own triangles (model-local indexing)
+    const uint32_t *mat_idx; // material of each triangle, for slot_nm
+    float4 *slot_nm;     // per triangle slot {geometric normal, material bits}, or null
     uint32_t W, leaf_max, node_bytes;
     uint32_t prim_base;  // added to the primitive index stored in a triangle slot (scene-global ids)
 };
@@ -722,6 +724,11 @@ __global__ void k_collapse_emit(Collapse C, const uint32_t *__restrict__ level, 
                         t[0] = make_float4(v[0], v[1], v[2], __uint_as_float(prim + C.prim_base));
                         t[1] = make_float4(v[3], v[4], v[5], 0.0f);
                         t[2] = make_float4(v[6], v[7], v[8], 0.0f);
+                        if (C.slot_nm) { // the normal as the shading forms it from the vertices
+                            const v3 a = mk(v[0], v[1], v[2]);
+                            const v3 n = normalize(cross(sub(mk(v[3], v[4], v[5]), a), sub(mk(v[6], v[7], v[8]), a)));
+                            C.slot_nm[tbase + toff] = make_float4(n.x, n.y, n.z, __uint_as_float(C.mat_idx[prim]));
+                        }
                         toff++;
                     } else {
                         st[sp++] = right_of(C.T, y);
@@ -796,6 +803,8 @@ struct BvhTarget {
     uint32_t n;
     float4 *nbox;        // binary nodes float4[2*max(1, n-1)]; nullptr = take them from the scratch
     uint32_t *order;     // uint32[n]: sorted primitive order (BVH-local indices)
+    const uint32_t *mat_idx; // uint32[n]: material of each triangle (with slot_nm)
+    float4 *slot_nm;     // normal and material per triangle slot; nullptr = not wanted
     uint8_t *wide;       // node array; this BVH's nodes start at node_base
     float4 *tris;        // triangle slot array; this BVH's slots start at slot_base
     uint32_t node_base, node_cap; // region of the node array reserved for this BVH
@@ -890,7 +899,7 @@ crg_status build_pipeline(const BvhTarget &t, const crg_build_opts &o, ScratchSo
     BP_CHECK(cudaGetLastError());
 
     // level-by-level collapse into the target region
-    Collapse Cc{Tr, t.verts, o.width, o.leaf_max, node_bytes, t.prim_base};
+    Collapse Cc{Tr, t.verts, t.mat_idx, t.slot_nm, o.width, o.leaf_max, node_bytes, t.prim_base};
     k_fill<<<1, 32, 0, st>>>(lvl0, 1, n >= 2 ? 0u : LEAF);
     uint32_t L = 1, node_start = 0, next_start = 1, tri_start = 0, depth = 0;
     uint32_t *cur = lvl0, *nxt = lvl1;
@@ -981,6 +990,8 @@ crg_status build_bvh(crg_scene *s, const crg_build_opts &o, cudaStream_t st) {
             return rc;
         if ((rc = grow_keep(ctx, s->tris, sizeof(float4) * 3 * s->ntri, sizeof(float4) * 3 * kept_prims, st)) != CRG_OK)
             return rc;
+        if ((rc = grow_keep(ctx, s->slot_nm, sizeof(float4) * s->ntri, sizeof(float4) * kept_prims, st)) != CRG_OK)
+            return rc;
         if (cap > old_cap || !same) // unused node slots read as zero (deterministic downloads)
             CRG_CUDA(ctx, cudaMemsetAsync((uint8_t *)s->wide.ptr + (size_t)s->node_bytes * keep_nodes, 0,
                                           (size_t)s->node_bytes * (cap - keep_nodes), st));
@@ -992,6 +1003,8 @@ crg_status build_bvh(crg_scene *s, const crg_build_opts &o, cudaStream_t st) {
                     m.ntri,
                     (float4 *)s->bvh2.ptr + 2 * (size_t)m.node_base,
                     (uint32_t *)s->order.ptr + m.first,
+                    (const uint32_t *)s->mat_idx.ptr + m.first,
+                    (float4 *)s->slot_nm.ptr,
                     (uint8_t *)s->wide.ptr,
                     (float4 *)s->tris.ptr,
                     m.node_base,
@@ -1140,7 +1153,7 @@ extern "C" crg_status crg_build_bvh_noalloc(const float *d_verts, uint32_t ntri,
     (void)cudaGetLastError();
     cudaStream_t st = (cudaStream_t)stream;
     FixedScratch src(base);
-    BvhTarget t{d_verts, n, nullptr, d_order, (uint8_t *)d_wide, (float4 *)d_tris, 0, nint, 0, 0};
+    BvhTarget t{d_verts, n, nullptr, d_order, nullptr, nullptr, (uint8_t *)d_wide, (float4 *)d_tris, 0, nint, 0, 0};
     BvhResult res;
     std::string msg;
     const crg_status rc = build_pipeline(t, o, src, st, res, &msg);

@@ -670,7 +670,7 @@ crg_status scene_common(crg_context *ctx, uint32_t ntri, const uint32_t *mat_idx
 void scene_free(crg_scene *s) {
     if (!s) return;
     DevBuf *bufs[] = {&s->verts, &s->mat_idx, &s->mats, &s->light_prim, &s->light_alias, &s->light_pdf, &s->mat_light_pdf,
-                      &s->sky, &s->bvh2, &s->order, &s->wide, &s->tris, &s->err, &s->counters, &s->qhead,
+                      &s->sky, &s->bvh2, &s->order, &s->wide, &s->tris, &s->slot_nm, &s->err, &s->counters, &s->qhead,
                       &s->uvs, &s->texels, &s->tex_info, &s->inst, &s->light_inst, &s->light_rec,
                       &s->inst_root, &s->tlas};
     for (DevBuf *b : bufs) dev_free(*b);

@@ -110,6 +110,7 @@ struct crg_scene {
     DevBuf order;  // uint32[ntri]: each model's sorted primitive order at first, model-local indices
     DevBuf wide;   // node_bytes * node_cap: each model's wide BVH at node_base (indices scene-global)
     DevBuf tris;   // float4[3*ntri]: each model's triangle slots at first (primitive ids scene-global)
+    DevBuf slot_nm; // float4[ntri] per triangle slot: geometric normal (object space), material index bits
     DevBuf err;    // uint32 device error word
     DevBuf qhead;  // uint32 work counter of the persistent query kernels
     // statistics

@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(128) k_draft(SceneDev S, CamDev cam, uint32_t 
     float4 c;
     if (found) {
         const HitGeom g = hit_geom<false>(S, h, o, d);
-        const crg_material &m = S.mats[__ldg(&S.mat_idx[h.prim])];
+        const crg_material &m = S.mats[g.mat];
         const float4 col = hit_colour(S, m, h.prim, h.slot, g.ro, g.rd);
         c = textured(S, m) ? col : make_float4(col.x, col.y, col.z, 1.0f);
     } else {

@@ -225,6 +225,7 @@ SceneDev scene_dev(const crg_scene *s) {
     SceneDev S{};
     S.nodes = (const uint4 *)s->wide.ptr;
     S.tris = (const float4 *)s->tris.ptr;
+    S.slot_nm = (const float4 *)s->slot_nm.ptr;
     S.mat_idx = (const uint32_t *)s->mat_idx.ptr;
     S.mats = (const crg_material *)s->mats.ptr;
     S.light_prim = (const uint32_t *)s->light_prim.ptr;
