@@ -21,8 +21,9 @@
 // ray, throughput and radiance.  The traversal stages refill idle lanes ray
 // by ray and trace a ray through a scene's placements themselves.
 //
-// extend / shade / shadow are persistent kernels: a fixed grid whose warps
-// take `fetch` queue entries at a time with one atomic.  The order in which L
+// extend / shade / shadow are persistent kernels on a fixed grid; without
+// refill, the traversal stages' warps take `fetch` queue entries at a time
+// with one atomic.  The order in which L
 // receives contributions (emission of bounce i, then NEE of bounce i, then
 // bounce i + 1) is the megakernel's, because the shadow kernel of bounce i
 // runs before the shade kernel of bounce i + 1.
@@ -63,7 +64,8 @@ struct Chunk {
 };
 
 struct Ctrl {
-    unsigned int in_count, out_count, sh_count;
+    unsigned long long pushed; // entries of the output queue (low 32 bits) and of the shadow queue (high)
+    unsigned int in_count;
     unsigned int head_ext, head_shade, head_sh;
     unsigned int parity;
     unsigned int chunk;          // chunk being rendered
@@ -107,6 +109,8 @@ __device__ __forceinline__ float pack_found(bool found, uint32_t inst) {
     return __uint_as_float(found ? (inst == kNoInst ? 1u : inst + 2u) : 0u);
 }
 
+__device__ __forceinline__ unsigned int sh_count(const Ctrl *c) { return (unsigned int)(c->pushed >> 32); }
+
 __device__ __forceinline__ uint32_t *q_in(const Wf &w, const Ctrl &c) { return c.parity ? w.qb : w.qa; }
 __device__ __forceinline__ uint32_t *q_out(const Wf &w, const Ctrl &c) { return c.parity ? w.qa : w.qb; }
 
@@ -118,15 +122,15 @@ __device__ __forceinline__ unsigned int warp_fetch(unsigned int *head, uint32_t 
     return __shfl_sync(0xFFFFFFFFu, b, 0);
 }
 
-// Warp-aggregated append of flagged lanes to a queue.
-__device__ __forceinline__ void warp_push(bool want, uint32_t value, uint32_t *queue, unsigned int *count) {
+// Warp-aggregated append of flagged lanes to the output queue.
+__device__ __forceinline__ void warp_push(bool want, uint32_t value, uint32_t *queue, Ctrl *c) {
     const uint32_t active = __activemask();
     const uint32_t m = __ballot_sync(active, want);
     if (!m) return;
     const uint32_t lane = threadIdx.x & 31;
     const int leader = __ffs(m) - 1;
     unsigned int base = 0;
-    if ((int)lane == leader) base = atomicAdd(count, (unsigned int)__popc(m));
+    if ((int)lane == leader) base = (unsigned int)atomicAdd(&c->pushed, (unsigned long long)__popc(m));
     base = __shfl_sync(active, base, leader);
     if (want) queue[base + __popc(m & ((1u << lane) - 1u))] = value;
 }
@@ -175,27 +179,32 @@ __device__ void start_sample(const Wf &w, uint32_t slot, unsigned long long gid,
     w.meta[slot] = make_uint4(sg.view | kPrevDelta | kFresh, pix, sample, (uint32_t)(gid - ch.gid_begin));
 }
 
+// Whether the chunk may have samples left to issue (read when a stage starts).
+// Its counter only grows, so a chunk that fits the pool is closed from the
+// start and its finished paths touch no counter.
+__device__ __forceinline__ bool samples_open(const Wf &w, const Ctrl *c) {
+    return *(const volatile unsigned long long *)&c->issued < w.chunks[c->chunk].gid_end;
+}
+
 // Writes a finished sample and, if the chunk has more, starts the next one
-// in the same slot (pushed to the output queue).
-__device__ __forceinline__ void finish_and_refill(const Wf &w, Ctrl *c, bool finishing, uint32_t slot, float4 Lv,
+// in the same slot (pushed to the output queue).  `open`: samples_open.
+__device__ __forceinline__ void finish_and_refill(const Wf &w, Ctrl *c, bool open, bool finishing, uint32_t slot, float4 Lv,
                                                   uint32_t off) {
     if (finishing) w.slots[off] = Lv;
+    if (!open) return;
     const uint32_t active = __activemask();
     const uint32_t m = __ballot_sync(active, finishing);
-    bool refill = false;
-    unsigned long long gid = 0;
+    if (!m) return;
     const Chunk ch = w.chunks[c->chunk];
-    if (m) {
-        const uint32_t lane = threadIdx.x & 31;
-        const int leader = __ffs(m) - 1;
-        unsigned long long base = 0;
-        if ((int)lane == leader) base = atomicAdd(&c->issued, (unsigned long long)__popc(m));
-        base = __shfl_sync(active, base, leader);
-        gid = base + __popc(m & ((1u << lane) - 1u));
-        refill = finishing && gid < ch.gid_end;
-    }
+    const uint32_t lane = threadIdx.x & 31;
+    const int leader = __ffs(m) - 1;
+    unsigned long long base = 0;
+    if ((int)lane == leader) base = atomicAdd(&c->issued, (unsigned long long)__popc(m));
+    base = __shfl_sync(active, base, leader);
+    const unsigned long long gid = base + __popc(m & ((1u << lane) - 1u));
+    const bool refill = finishing && gid < ch.gid_end;
     if (refill) start_sample(w, slot, gid, ch);
-    warp_push(refill, slot, q_out(w, *c), &c->out_count);
+    warp_push(refill, slot, q_out(w, *c), c);
 }
 
 template <int W, bool CNT, bool INST>
@@ -233,13 +242,13 @@ __global__ void __launch_bounds__(256) k_wf_extend(Wf w) {
     }
 }
 
-// Warp-aggregated count of flagged lanes (shadow rays traced inside a fused shade kernel).
-__device__ __forceinline__ void warp_count(bool want, unsigned int *count) {
-    const uint32_t active = __activemask();
-    const uint32_t m = __ballot_sync(active, want);
-    if (m && (threadIdx.x & 31) == (uint32_t)(__ffs(m) - 1)) atomicAdd(count, (unsigned int)__popc(m));
-}
-
+// One bounce of every queued path.  A warp takes rows of 32 entries, by its place
+// in the grid where only shading is done (the entries' work is alike), else
+// `fetch` entries per atomic, and reserves its places in the two
+// queues by one atomic: the counters are single addresses for the whole GPU,
+// and at four atomics a warp (fetch, two pushes, samples issued) they held the
+// stage to 104 ms of the ten-view batch's frame, against 53 ms now (32, 128 or
+// 256 entries to a reservation: 52.6 / 53.7 / 52.8 ms).
 // FUSE 0: shade only (hits from k_wf_extend, shadow rays to the shadow queue)
 // FUSE 1: shade + the NEE shadow test in the same thread (no shadow queue)
 // FUSE 2: closest hit + shade + shadow test (one kernel per bounce)
@@ -251,100 +260,112 @@ __global__ void __launch_bounds__(256, FUSE == 0 ? 3 : 2) k_wf_shade(Wf w) {
     Ctrl *c = w.ctrl;
     const unsigned int n = c->in_count;
     const uint32_t *in = q_in(w, *c);
+    uint32_t *out = q_out(w, *c);
+    const bool open = samples_open(w, c);
     const uint32_t lane = threadIdx.x & 31;
-    for (;;) {
-        const unsigned int base = warp_fetch(&c->head_shade, w.fetch);
-        if (base >= n) break;
-        for (uint32_t k0 = 0; k0 < w.fetch; k0 += 32) {
-            if (base + k0 >= n) break;
-            const unsigned int qi = base + k0 + lane;
-            const bool valid = qi < n && k0 + lane < w.fetch;
-            uint32_t slot = 0;
-            bool cont = false, finishing = false, shadow = false;
-            float4 Lv = make_float4(0, 0, 0, 0);
-            uint32_t off = 0;
-            if (valid) {
-                slot = in[qi];
-                uint4 m = w.meta[slot];
-                const uint32_t view = m.x & 0xFFFFu, depth = (m.x >> 16) & 0x3FFu;
-                const ViewDev &V = w.views[view];
-                const SceneDev &S = w.scenes[V.scene];
-                float4 o, d, T, L;
-                path_ray(w, slot, m, o, d);
-                if (m.x & kFresh) {
-                    T = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
-                    L = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                } else {
-                    T = w.T[slot];
-                    L = w.L[slot];
-                }
-                PathCtx C{m.y, m.z, V.set.seed, 0, 0, 0, 0ull, 0ull};
-                float4 h4;
-                if (FUSE >= 2) {
-                    Hit hh;
-                    const bool f = closest<W, CNT, INST>(S, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), INFINITY, hh, C);
-                    h4 = make_float4(hh.t, __uint_as_float(hh.prim), __uint_as_float(hh.slot), pack_found(f, hh.inst));
-                } else {
-                    h4 = w.hit[slot];
-                }
-                PathState ps;
-                ps.o = mk(o.x, o.y, o.z);
-                ps.d = mk(d.x, d.y, d.z);
-                ps.T = mk(T.x, T.y, T.z);
-                ps.L = mk(L.x, L.y, L.z);
-                ps.prev_pdf = T.w;
-                ps.prev_delta = (m.x & kPrevDelta) ? 1u : 0u;
-                Hit h;
-                h.t = h4.x;
-                h.prim = __float_as_uint(h4.y);
-                h.slot = __float_as_uint(h4.z);
-                h.u = h.v = 0.0f;
-                const uint32_t fw = __float_as_uint(h4.w);
-                h.inst = fw >= 2u ? fw - 2u : kNoInst;
-                Aov aov;
-                NeeReq nr;
-                nr.kind = 0;
-                if (depth >= V.set.max_bounces) {
-                    cont = false; // max_bounces == 0: the megakernel traces nothing for this sample
-                } else {
-                    cont = V.set.mode == CRG_MODE_EXTENDED
-                               ? shade_extended(S, V.set, C, depth, ps, fw != 0u, h, aov, nr)
-                               : shade_faithful(S, V.set, C, depth, ps, fw != 0u, h, aov, nr);
-                }
-                if (cont && depth + 1 >= V.set.max_bounces) cont = false;
-                shadow = nr.kind != 0;
-                if (FUSE >= 1 && shadow && shadow_visible<W, CNT, INST>(S, nr, C)) ps.L = add(ps.L, nr.c);
-                if (C.err) atomicOr(&c->error, 1u);
-                if (CNT) {
-                    nodes += C.nodes;
-                    tris += C.tris;
-                }
-                Lv = make_float4(ps.L.x, ps.L.y, ps.L.z, 0.0f);
-                off = m.w;
-                finishing = !cont && (FUSE >= 1 || !shadow);
-                if (FUSE == 0 && shadow) {
-                    w.sh_o[slot] = make_float4(nr.o.x, nr.o.y, nr.o.z, nr.tmax);
-                    w.sh_d[slot] = make_float4(nr.d.x, nr.d.y, nr.d.z, __uint_as_float(nr.kind));
-                    w.sh_c[slot] = make_float4(nr.c.x, nr.c.y, nr.c.z, 0.0f);
-                }
-                uint32_t mx_ = (m.x & 0xFFFFu) | ((depth + 1) << 16) | (ps.prev_delta ? kPrevDelta : 0u);
-                if (FUSE == 0 && !cont && shadow) mx_ |= kFinish;
-                m.x = mx_;
-                if (!finishing) { // a finishing path's radiance goes to its sample slot; its state is dead
-                    w.L[slot] = Lv;
-                    w.meta[slot] = m;
-                }
-                if (cont) {
-                    w.o[slot] = make_float4(ps.o.x, ps.o.y, ps.o.z, 0.0f);
-                    w.d[slot] = make_float4(ps.d.x, ps.d.y, ps.d.z, 0.0f);
-                    w.T[slot] = make_float4(ps.T.x, ps.T.y, ps.T.z, ps.prev_pdf);
-                }
-            }
-            if (FUSE == 0) warp_push(valid && shadow, slot, w.qsh, &c->sh_count);
-            else warp_count(valid && shadow, &c->sh_count);
-            warp_push(valid && cont, slot, q_out(w, *c), &c->out_count);
-            finish_and_refill(w, c, valid && finishing, slot, Lv, off);
+    unsigned int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
+    for (uint32_t left = 0;; left -= 32) {
+        if (FUSE >= 1 && left == 0) {
+            base = warp_fetch(&c->head_shade, w.fetch);
+            left = w.fetch;
         }
+        if (base >= n) break;
+        const unsigned int qi = base + lane;
+        const bool valid = qi < n;
+        uint32_t slot = 0;
+        bool cont = false, finishing = false, shadow = false;
+        float4 Lv = make_float4(0, 0, 0, 0);
+        uint32_t off = 0;
+        if (valid) {
+            slot = in[qi];
+            uint4 m = w.meta[slot];
+            const uint32_t view = m.x & 0xFFFFu, depth = (m.x >> 16) & 0x3FFu;
+            const ViewDev &V = w.views[view];
+            const SceneDev &S = w.scenes[V.scene];
+            float4 o, d, T, L;
+            path_ray(w, slot, m, o, d);
+            if (m.x & kFresh) {
+                T = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+                L = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            } else {
+                T = w.T[slot];
+                L = w.L[slot];
+            }
+            PathCtx C{m.y, m.z, V.set.seed, 0, 0, 0, 0ull, 0ull};
+            float4 h4;
+            if (FUSE >= 2) {
+                Hit hh;
+                const bool f = closest<W, CNT, INST>(S, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), INFINITY, hh, C);
+                h4 = make_float4(hh.t, __uint_as_float(hh.prim), __uint_as_float(hh.slot), pack_found(f, hh.inst));
+            } else {
+                h4 = w.hit[slot];
+            }
+            PathState ps;
+            ps.o = mk(o.x, o.y, o.z);
+            ps.d = mk(d.x, d.y, d.z);
+            ps.T = mk(T.x, T.y, T.z);
+            ps.L = mk(L.x, L.y, L.z);
+            ps.prev_pdf = T.w;
+            ps.prev_delta = (m.x & kPrevDelta) ? 1u : 0u;
+            Hit h;
+            h.t = h4.x;
+            h.prim = __float_as_uint(h4.y);
+            h.slot = __float_as_uint(h4.z);
+            h.u = h.v = 0.0f;
+            const uint32_t fw = __float_as_uint(h4.w);
+            h.inst = fw >= 2u ? fw - 2u : kNoInst;
+            Aov aov;
+            NeeReq nr;
+            nr.kind = 0;
+            if (depth >= V.set.max_bounces) {
+                cont = false; // max_bounces == 0: the megakernel traces nothing for this sample
+            } else {
+                cont = V.set.mode == CRG_MODE_EXTENDED
+                           ? shade_extended(S, V.set, C, depth, ps, fw != 0u, h, aov, nr)
+                           : shade_faithful(S, V.set, C, depth, ps, fw != 0u, h, aov, nr);
+            }
+            if (cont && depth + 1 >= V.set.max_bounces) cont = false;
+            shadow = nr.kind != 0;
+            if (FUSE >= 1 && shadow && shadow_visible<W, CNT, INST>(S, nr, C)) ps.L = add(ps.L, nr.c);
+            if (C.err) atomicOr(&c->error, 1u);
+            if (CNT) {
+                nodes += C.nodes;
+                tris += C.tris;
+            }
+            Lv = make_float4(ps.L.x, ps.L.y, ps.L.z, 0.0f);
+            off = m.w;
+            finishing = !cont && (FUSE >= 1 || !shadow);
+            if (FUSE == 0 && shadow) {
+                w.sh_o[slot] = make_float4(nr.o.x, nr.o.y, nr.o.z, nr.tmax);
+                w.sh_d[slot] = make_float4(nr.d.x, nr.d.y, nr.d.z, __uint_as_float(nr.kind));
+                w.sh_c[slot] = make_float4(nr.c.x, nr.c.y, nr.c.z, 0.0f);
+            }
+            uint32_t mx_ = (m.x & 0xFFFFu) | ((depth + 1) << 16) | (ps.prev_delta ? kPrevDelta : 0u);
+            if (FUSE == 0 && !cont && shadow) mx_ |= kFinish;
+            m.x = mx_;
+            if (!finishing) { // a finishing path's radiance goes to its sample slot; its state is dead
+                w.L[slot] = Lv;
+                w.meta[slot] = m;
+            }
+            if (cont) {
+                w.o[slot] = make_float4(ps.o.x, ps.o.y, ps.o.z, 0.0f);
+                w.d[slot] = make_float4(ps.d.x, ps.d.y, ps.d.z, 0.0f);
+                w.T[slot] = make_float4(ps.T.x, ps.T.y, ps.T.z, ps.prev_pdf);
+            }
+        }
+        // one reservation in both queues for the warp
+        const uint32_t mo = __ballot_sync(0xFFFFFFFFu, cont), ms = __ballot_sync(0xFFFFFFFFu, shadow);
+        if (mo | ms) {
+            unsigned long long at = 0;
+            if (lane == 0)
+                at = atomicAdd(&c->pushed, (unsigned long long)__popc(mo) | (unsigned long long)__popc(ms) << 32);
+            at = __shfl_sync(0xFFFFFFFFu, at, 0);
+            const uint32_t lt = (1u << lane) - 1u;
+            if (cont) out[(uint32_t)at + __popc(mo & lt)] = slot;
+            if (FUSE == 0 && shadow) w.qsh[(uint32_t)(at >> 32) + __popc(ms & lt)] = slot;
+        }
+        finish_and_refill(w, c, open, finishing, slot, Lv, off);
+        base += FUSE == 0 ? gridDim.x * blockDim.x : 32u;
     }
     if (CNT && FUSE >= 1) { // FUSE 1: the shadow test's work; FUSE 2: closest hit and shadow test together
         atomicAdd(FUSE == 1 ? &c->nodes_sh : &c->nodes, nodes);
@@ -356,7 +377,8 @@ template <int W, bool CNT, bool INST>
 __global__ void __launch_bounds__(256) k_wf_shadow(Wf w) {
     unsigned long long nodes = 0, tris = 0;
     Ctrl *c = w.ctrl;
-    const unsigned int n = c->sh_count;
+    const unsigned int n = sh_count(c);
+    const bool open = samples_open(w, c);
     const uint32_t lane = threadIdx.x & 31;
     for (;;) {
         const unsigned int base = warp_fetch(&c->head_sh, w.fetch);
@@ -395,7 +417,7 @@ __global__ void __launch_bounds__(256) k_wf_shadow(Wf w) {
                 finishing = (m.x & kFinish) != 0u;
                 off = m.w;
             }
-            finish_and_refill(w, c, valid && finishing, slot, Lv, off);
+            finish_and_refill(w, c, open, valid && finishing, slot, Lv, off);
         }
     }
     if (CNT) {
@@ -533,7 +555,8 @@ __global__ void __launch_bounds__(256, 4) k_wf_extend_dyn(Wf w) {
 template <int W, bool CNT, int PL>
 __global__ void __launch_bounds__(256, 4) k_wf_shadow_dyn(Wf w) {
     Ctrl *c = w.ctrl;
-    const unsigned int n = c->sh_count;
+    const unsigned int n = sh_count(c);
+    const bool open = samples_open(w, c);
     TravStats st{0, 0};
     uint32_t err = 0;
     const SceneDev *Sp = nullptr;
@@ -609,7 +632,7 @@ __global__ void __launch_bounds__(256, 4) k_wf_shadow_dyn(Wf w) {
                 Lv = make_float4(L.x, L.y, L.z, 0.0f);
                 w.L[slot] = Lv;
             }
-            finish_and_refill(w, c, (m.x & kFinish) != 0u, slot, Lv, m.w);
+            finish_and_refill(w, c, open, (m.x & kFinish) != 0u, slot, Lv, m.w);
         },
         st, err);
     if (err) atomicOr(&c->error, 1u);
@@ -629,11 +652,10 @@ __global__ void k_wf_control(Wf w, cudaGraphConditionalHandle handle, int in_gra
         return;
     }
     c->segments += c->in_count;
-    c->shadow += c->sh_count;
+    c->shadow += sh_count(c);
     c->parity ^= 1u;
-    c->in_count = c->out_count;
-    c->out_count = 0;
-    c->sh_count = 0;
+    c->in_count = (unsigned int)c->pushed;
+    c->pushed = 0;
     c->head_ext = c->head_shade = c->head_sh = 0;
     c->resolve_chunk = 0xFFFFFFFFu;
     c->generate = 0;

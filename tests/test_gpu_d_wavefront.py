@@ -376,3 +376,22 @@ def test_small_batch_call_overhead(ctx, capsys):
     assert enq_us < sync_us
     f.close()
     s.close()
+
+
+@pytest.mark.parametrize("size,spp", [((1, 1), 1), ((31, 1), 1), ((33, 1), 3), ((37, 29), 5)])
+@pytest.mark.parametrize("opts", [None, dict(path_pool=33), dict(path_pool=100, refill=OFF), dict(fuse=2, fetch=64),
+                                  dict(path_pool=64, fuse=3, fetch=96)])
+def test_queue_edges_match_megakernel(ctx, size, spp, opts):
+    """Queues of a few entries, pools that are no multiple of a warp, and chunks
+    larger than the pool (finished paths take the next samples) or not."""
+    sc = _box_variant("materials")
+    s = api.Scene(ctx, sc["verts"], sc["mat_idx"], sc["mats"]).build()
+    st = api.make_settings(size[0], size[1], spp, max_bounces=8, rr_depth=3, mode=1, seed=31, aspect=size[0] / size[1])
+    try:
+        ref = _mega(ctx, s, sc["camera"], st)
+        f = api.Film(ctx, size[0], size[1], f64=True)
+        ctx.check(api.render_batch([s], [(0, sc["camera"], st)], [f], opts))
+        _same(f.download(f64=True), ref)
+        f.close()
+    finally:
+        s.close()
