@@ -363,7 +363,7 @@ const char *crg_noalloc_last_error(void);
  *   info       : optional; filled like crg_scene_bvh_info
  *
  * Scratch (sort keys, tree arrays, collapse levels) lives in one fixed device
- * array inside the library, about 2.5 MB, which every GPU that loads the
+ * array inside the library, about 3 MB, which every GPU that loads the
  * library holds until the process exits.  All calls share it and it keeps the
  * last call's contents: the call clears what must start at zero, but two calls
  * whose work overlaps on the GPU (different streams or threads at once) race

@@ -71,3 +71,20 @@ def test_empty_scene_builds(ctx):
         assert (s.intersect(rays, any_hit=True) == 0).all()
     finally:
         s.close()
+
+
+@pytest.mark.parametrize("n", [7, 8, 13, 14, 15, 27, 28, 29, 33, 64, 257])
+@pytest.mark.parametrize("rounds", [1, 3, 8])
+def test_treelet_edges_bit_exact(ctx, orc, n, rounds):
+    """Treelet rounds on trees at the edges of the rounds' leaf counts (7, 14, 28, ...)
+    and of a warp's 32 leaves."""
+    v = np.ascontiguousarray(scenes.soup(n, 60 + n, 0.1))
+    s = api.Scene(ctx, v, np.zeros(n, np.uint32), _mats()).build(8, 1, 2, rounds)
+    try:
+        gi, g = s.info(), s.download_bvh()
+    finally:
+        s.close()
+    o = orc.Bvh(v, width=8, treelet=1, leaf_max=2, rounds=rounds)
+    assert gi == o.info()
+    for a, b in zip(g, o.download()):
+        assert np.array_equal(a.view(np.uint8), b.view(np.uint8))
