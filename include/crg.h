@@ -363,7 +363,7 @@ const char *crg_noalloc_last_error(void);
  *   info       : optional; filled like crg_scene_bvh_info
  *
  * Scratch (sort keys, tree arrays, collapse levels) lives in one fixed device
- * array inside the library, about 3 MB, which every GPU that loads the
+ * array inside the library, about 2.5 MB, which every GPU that loads the
  * library holds until the process exits.  All calls share it and it keeps the
  * last call's contents: the call clears what must start at zero, but two calls
  * whose work overlaps on the GPU (different streams or threads at once) race
@@ -373,7 +373,7 @@ const char *crg_noalloc_last_error(void);
  * context was created on — that first call may load the library's device code
  * and reserve the array (a driver-side allocation and a synchronisation), so
  * make it before any stream capture, or create a context on the device first.
- * The call synchronises `stream` once per BVH level, as crg_scene_build does;
+ * The call synchronises `stream` before it returns, as crg_scene_build does;
  * when it fails after queueing work it waits for that work to finish before
  * returning.  Errors are described by crg_noalloc_last_error. */
 crg_status crg_build_bvh_noalloc(const float *d_verts, uint32_t ntri, const crg_build_opts *opts,
