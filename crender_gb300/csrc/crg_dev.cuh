@@ -600,6 +600,45 @@ __device__ __forceinline__ void lane_visit(LaneTrav &T, uint2 *stack, const uint
     if (T.ng.y < 1u << 24 && T.sp > 0) T.ng = stack[--T.sp];
 }
 
+// Traversal of one ray per lane by a whole warp, to completion: lanes with `on`
+// trace the ray r (its box half is taken over, its triangle half stored), the
+// others only test triangles.  ANY as a run-time switch (the same for the whole
+// warp): a ray ends at its first hit below tmax, which best_prim then shows.
+template <int W, bool COUNT>
+__device__ __forceinline__ void warp_traverse(bool on, bool any, const RayPre &r, float tmax, uint32_t root,
+                                              const uint4 *__restrict__ nodes, const float4 *__restrict__ tris, WarpRays &sh,
+                                              LaneTrav &T, TravStats &st, uint32_t &err) {
+    constexpr uint32_t kVisitors = 16; // 8 / 16 / 24: mesh 14.36 / 14.46 / 14.57 ms, box 13.62 / 13.57 / 13.58
+    uint2 stack[kStack];
+    if (on) {
+        lane_init(T, r, tmax, root);
+        put_ray(sh, threadIdx.x & 31u, r, tris);
+    } else {
+        T.ng = T.tg = make_uint2(0u, 0u);
+    }
+    __syncwarp();
+    for (;;) {
+        const bool can = T.tg.y == 0u && T.ng.y >= 1u << 24;
+        const uint32_t visitors = __ballot_sync(0xFFFFFFFFu, can);
+        if ((uint32_t)__popc(visitors) < kVisitors) {
+            // few lanes to visit with: the triangle tests first, if there are any
+            if (__any_sync(0xFFFFFFFFu, T.tg.y != 0u)) {
+                warp_tris<false>(T, sh, tris);
+                if (any && on && T.best_prim != 0xFFFFFFFFu) T.ng.y = 0u;
+                continue;
+            }
+            if (visitors == 0u) return;
+        }
+        if (can) {
+            lane_visit<W>(T, stack, nodes, err);
+            if (COUNT) {
+                st.nodes++;
+                st.tris += (uint32_t)__popc(T.tg.y);
+            }
+        }
+    }
+}
+
 // Traversal of a queue of rays by a warp: node visits for as long as at least
 // VISITORS lanes have no triangles pending, then the pending triangles of all
 // lanes; one visit yields 0.55 triangles per ray on the soup, so a second visit

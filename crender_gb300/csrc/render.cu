@@ -52,119 +52,153 @@ using namespace rc;
 
 namespace {
 
-// MINB blocks of 128 threads per SM: 5 (96 registers, some spilled) when the grid fills the
-// GPU at that occupancy, else 4 (no spills: a grid below one wave gains nothing from the
-// extra warps and loses the spill traffic).
-// INST: the scene is traced through its placements (models and instances);
-// kernels for plain one-mesh scenes are compiled without that code.
-template <int W, int MODE, bool CNT, int MINB, bool INST>
+// MINB: blocks of 128 threads per SM, see launch_w.
+// PL: how the scene's placements are traced (warp_trace).
+//
+// A warp traces its lanes' segments together and then their shadow tests, sharing
+// the triangle tests (warp_traverse).  Both go through one place in the code, the
+// phase loop: the kernel is bound by instruction issue and fetch as much as by
+// divergence, and two copies of the traversal do not fit the instruction cache.
+// Lanes cover 8 x 4 pixel tiles (tile_pixel).  Against a traversal per thread on
+// rows of pixels: box 512x512x64 15.6 -> 12.7 ms (19.6 instead of 11.3 lanes
+// active), 4.2M-triangle mesh 1920x1080x4 15.5 -> 12.7, six placements with the
+// reference estimator 1283x721 1.99 -> 1.23.
+template <int W, int MODE, bool CNT, int MINB, int PL>
 __global__ void __launch_bounds__(128, MINB) k_render(SceneDev S, CamDev cam, crg_settings set, FilmDev F, uint64_t spp0) {
-    const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ WarpRays s_rays[4];
+    extern __shared__ double s_sums[]; // films with FP64 planes: 6 sums per thread
+    WarpRays &sh = s_rays[threadIdx.x >> 5];
+    const uint32_t place = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t Wd = set.width, Hd = set.height;
+    const bool inside = place < Wd * Hd;
+    // a grid below a wave runs row by row: its time is its slowest block's, and tiles make
+    // blocks less alike (256x256 box forward pass 3% slower with them)
+    const uint32_t pix = inside ? (PL == 0 && MINB == 4 ? place : tile_pixel(place, Wd, Hd)) : 0u;
     PathCtx C{pix, 0, set.seed, 0, 0, 0, 0ull, 0ull};
-    uint32_t lanes = __ballot_sync(0xFFFFFFFFu, pix < Wd * Hd);
-    if (pix < Wd * Hd) {
-        const uint32_t px = pix % Wd, py = pix / Wd;
-        const size_t fidx = (size_t)(Wd - 1 - px) + (size_t)(Hd - 1 - py) * Wd;
-        float acc[3] = {F.sum[fidx * 3], F.sum[fidx * 3 + 1], F.sum[fidx * 3 + 2]};
-        double a64[3] = {0, 0, 0}, q64[3] = {0, 0, 0};
-        if (F.sum64) {
-            a64[0] = F.sum64[fidx * 3]; a64[1] = F.sum64[fidx * 3 + 1]; a64[2] = F.sum64[fidx * 3 + 2];
-            q64[0] = F.sumsq64[fidx * 3]; q64[1] = F.sumsq64[fidx * 3 + 1]; q64[2] = F.sumsq64[fidx * 3 + 2];
-        }
-        Aov aov;
-        PathState ps;
-        // Path regeneration (Novak, Havran and Dachsbacher 2010): one loop over
-        // segments, in which a lane whose path has ended starts its pixel's next
-        // sample, so a warp runs for the largest total segment count of its lanes
-        // instead of the longest path of every sample.  A pixel's samples still run
-        // and accumulate in order, so the film is unchanged.
-        uint32_t s = 0, i = 0;
-        for (;;) {
-            // the lanes still rendering meet here before every segment, so the warp
-            // enters each segment's traversal together
-            lanes = __ballot_sync(lanes, s < set.spp);
-            if (s >= set.spp) break;
-            if (i == 0) {
-                C.sample = (uint32_t)(spp0 + s);
-                const f4 g0 = rand4(pix, C.sample, 0, set.seed);
-                const float x = ((float)px + g0.x) / (float)Wd;
-                const float y = ((float)py + g0.y) / (float)Hd;
-                v3 o, d;
-                camera_ray(cam, x, y, set.aspect, o, d);
-                aov.albedo = mk(0, 0, 0);
-                aov.normal = mk(0, 0, 0);
-                aov.depth = 0.0f;
-                path_start(ps, o, d);
+    const uint32_t px = pix % Wd, py = pix / Wd;
+    const size_t fidx = inside ? (size_t)(Wd - 1 - px) + (size_t)(Hd - 1 - py) * Wd : 0;
+    float acc[3] = {0.0f, 0.0f, 0.0f};
+    if (inside) {
+        for (int k = 0; k < 3; ++k) acc[k] = F.sum[fidx * 3 + k];
+        if (F.sum64)
+            for (int k = 0; k < 3; ++k) {
+                s_sums[k * 128 + threadIdx.x] = F.sum64[fidx * 3 + k];
+                s_sums[(3 + k) * 128 + threadIdx.x] = F.sumsq64[fidx * 3 + k];
             }
-            if (i < set.max_bounces) {
-                Hit h;
+    }
+    PathState ps;
+    path_start(ps, mk(0, 0, 0), mk(0, 0, 1));
+    // Path regeneration (Novak, Havran and Dachsbacher 2010): one loop over
+    // segments, in which a lane whose path has ended starts its pixel's next
+    // sample, so a warp runs for the largest total segment count of its lanes
+    // instead of the longest path of every sample.  A pixel's samples still run
+    // and accumulate in order, so the film is unchanged.
+    uint32_t s = inside ? 0u : set.spp, i = 0;
+    while (__any_sync(0xFFFFFFFFu, s < set.spp)) {
+        const bool alive = s < set.spp;
+        if (alive && i == 0) {
+            C.sample = (uint32_t)(spp0 + s);
+            const f4 g0 = rand4(pix, C.sample, 0, set.seed);
+            const float x = ((float)px + g0.x) / (float)Wd;
+            const float y = ((float)py + g0.y) / (float)Hd;
+            v3 o, d;
+            camera_ray(cam, x, y, set.aspect, o, d);
+            path_start(ps, o, d);
+        }
+        const bool seg = alive && i < set.max_bounces;
+        bool cont = false;
+        Aov aov{mk(0, 0, 0), mk(0, 0, 0), 0.0f};
+        NeeReq nr;
+        nr.kind = 0;
+#pragma unroll 1
+        for (bool shadow = false;; shadow = true) {
+            const bool on = shadow ? nr.kind != 0 : seg;
+            if (shadow && !__any_sync(0xFFFFFFFFu, on)) break;
+            Hit h;
+            const v3 o = shadow ? nr.o : ps.o, d = shadow ? nr.d : ps.d;
+            warp_trace<W, CNT, PL>(S, sh, on, shadow && MODE == CRG_MODE_EXTENDED, o, d, shadow ? nr.tmax : INFINITY, h, C);
+            const bool found = h.prim != 0xFFFFFFFFu;
+            if (!on) continue;
+            if (!shadow) {
                 C.segments++;
-                const bool found = closest<W, CNT, INST>(S, ps.o, ps.d, INFINITY, h, C);
-                NeeReq nr;
-                const bool cont = MODE == CRG_MODE_EXTENDED ? shade_extended(S, set, C, i, ps, found, h, aov, nr)
-                                                            : shade_faithful(S, set, C, i, ps, found, h, aov, nr);
-                if (nr.kind != 0 && shadow_visible<W, CNT, INST>(S, nr, C)) ps.L = add(ps.L, nr.c);
-                ++i;
-                if (cont && i < set.max_bounces) continue;
+                cont = MODE == CRG_MODE_EXTENDED ? shade_extended(S, set, C, i, ps, found, h, aov, nr)
+                                                 : shade_faithful(S, set, C, i, ps, found, h, aov, nr);
+                continue;
             }
-            ++s;
-            i = 0;
-            const v3 L = ps.L;
-            acc[0] += L.x;
-            acc[1] += L.y;
-            acc[2] += L.z;
-            if (F.sum64) {
-                a64[0] += (double)L.x; a64[1] += (double)L.y; a64[2] += (double)L.z;
-                q64[0] += (double)L.x * (double)L.x;
-                q64[1] += (double)L.y * (double)L.y;
-                q64[2] += (double)L.z * (double)L.z;
+            C.shadow++;
+            nr.kind = 0;
+            if (!found) {
+                ps.L = add(ps.L, nr.c);
+            } else if (MODE == CRG_MODE_FAITHFUL) {
+                // the sun test steps 0.1 past alpha-zero surfaces (renderer.cpp:330-345)
+                const HitGeom hg = hit_geom<false>(S, h, o, d);
+                if (hit_colour(S, S.mats[hg.mat], h.prim, h.slot, hg.ro, hg.rd).w == 0.0f) {
+                    nr.o = add(hg.p, mul(nr.d, 0.1f));
+                    nr.kind = 2;
+                }
             }
         }
-        F.sum[fidx * 3] = acc[0];
-        F.sum[fidx * 3 + 1] = acc[1];
-        F.sum[fidx * 3 + 2] = acc[2];
-        if (F.sum64) {
-            F.sum64[fidx * 3] = a64[0]; F.sum64[fidx * 3 + 1] = a64[1]; F.sum64[fidx * 3 + 2] = a64[2];
-            F.sumsq64[fidx * 3] = q64[0]; F.sumsq64[fidx * 3 + 1] = q64[1]; F.sumsq64[fidx * 3 + 2] = q64[2];
-        }
-        if (F.aov_albedo && set.spp > 0) {
+        if (!alive) continue;
+        if (i == 0 && s + 1 == set.spp && F.aov_albedo) { // the last sample's first hit stays
             reinterpret_cast<float4 *>(F.aov_albedo)[fidx] = make_float4(aov.albedo.x, aov.albedo.y, aov.albedo.z, 1.0f);
             reinterpret_cast<float4 *>(F.aov_normal)[fidx] =
                 make_float4(aov.normal.x * 0.5f + 0.5f, aov.normal.y * 0.5f + 0.5f, aov.normal.z * 0.5f + 0.5f, 1.0f);
             const float dv = mn(aov.depth, 200.0f) / 200.0f;
             reinterpret_cast<float4 *>(F.aov_depth)[fidx] = make_float4(dv, dv, dv, 1.0f);
         }
+        if (seg && cont && ++i < set.max_bounces) continue;
+        ++s;
+        i = 0;
+        const v3 L = ps.L;
+        acc[0] += L.x;
+        acc[1] += L.y;
+        acc[2] += L.z;
+        if (F.sum64) {
+            double *q = s_sums + threadIdx.x;
+            q[0] += (double)L.x; q[128] += (double)L.y; q[256] += (double)L.z;
+            q[384] += (double)L.x * (double)L.x;
+            q[512] += (double)L.y * (double)L.y;
+            q[640] += (double)L.z * (double)L.z;
+        }
+    }
+    if (inside) {
+        for (int k = 0; k < 3; ++k) F.sum[fidx * 3 + k] = acc[k];
+        if (F.sum64)
+            for (int k = 0; k < 3; ++k) {
+                F.sum64[fidx * 3 + k] = s_sums[k * 128 + threadIdx.x];
+                F.sumsq64[fidx * 3 + k] = s_sums[(3 + k) * 128 + threadIdx.x];
+            }
     }
     if (C.err) atomicOr(S.err, C.err);
     if (CNT) {
-        unsigned long long seg = C.segments, sh = C.shadow, nd = C.nodes, tr = C.tris;
+        unsigned long long seg = C.segments, shr = C.shadow, nd = C.nodes, tr = C.tris;
 #pragma unroll
         for (int off = 16; off >= 1; off >>= 1) {
             seg += __shfl_xor_sync(0xFFFFFFFFu, seg, off);
-            sh += __shfl_xor_sync(0xFFFFFFFFu, sh, off);
+            shr += __shfl_xor_sync(0xFFFFFFFFu, shr, off);
             nd += __shfl_xor_sync(0xFFFFFFFFu, nd, off);
             tr += __shfl_xor_sync(0xFFFFFFFFu, tr, off);
         }
         if ((threadIdx.x & 31) == 0) {
             atomicAdd(&S.counters[1], seg);
-            atomicAdd(&S.counters[2], sh);
+            atomicAdd(&S.counters[2], shr);
             atomicAdd(&S.counters[3], nd);
             atomicAdd(&S.counters[4], tr);
         }
     }
 }
 
-template <int W, int MINB, bool INST>
+template <int W, int MINB, int PL>
 void launch_m(const SceneDev &S, const CamDev &cam, const crg_settings &set, const FilmDev &F, uint64_t spp0,
               uint32_t blocks, cudaStream_t st) {
     const uint32_t T = 128;
+    const size_t sums = F.sum64 ? sizeof(double) * 6 * T : 0;
     if (S.counters) {
-        if (set.mode == CRG_MODE_EXTENDED) k_render<W, CRG_MODE_EXTENDED, true, MINB, INST><<<blocks, T, 0, st>>>(S, cam, set, F, spp0);
-        else k_render<W, CRG_MODE_FAITHFUL, true, MINB, INST><<<blocks, T, 0, st>>>(S, cam, set, F, spp0);
+        if (set.mode == CRG_MODE_EXTENDED) k_render<W, CRG_MODE_EXTENDED, true, MINB, PL><<<blocks, T, sums, st>>>(S, cam, set, F, spp0);
+        else k_render<W, CRG_MODE_FAITHFUL, true, MINB, PL><<<blocks, T, sums, st>>>(S, cam, set, F, spp0);
     } else {
-        if (set.mode == CRG_MODE_EXTENDED) k_render<W, CRG_MODE_EXTENDED, false, MINB, INST><<<blocks, T, 0, st>>>(S, cam, set, F, spp0);
-        else k_render<W, CRG_MODE_FAITHFUL, false, MINB, INST><<<blocks, T, 0, st>>>(S, cam, set, F, spp0);
+        if (set.mode == CRG_MODE_EXTENDED) k_render<W, CRG_MODE_EXTENDED, false, MINB, PL><<<blocks, T, sums, st>>>(S, cam, set, F, spp0);
+        else k_render<W, CRG_MODE_FAITHFUL, false, MINB, PL><<<blocks, T, sums, st>>>(S, cam, set, F, spp0);
     }
 }
 
@@ -173,9 +207,16 @@ void launch_w(const SceneDev &S, const CamDev &cam, const crg_settings &set, con
               int sm_count, cudaStream_t st) {
     const uint64_t npix = (uint64_t)set.width * set.height;
     const uint32_t blocks = (uint32_t)((npix + 127) / 128);
-    if (S.ninst > kLoopPlacements) launch_m<W, 4, true>(S, cam, set, F, spp0, blocks, st); // the top-level tree
-    else if ((uint64_t)blocks >= 5ull * (uint64_t)(sm_count > 0 ? sm_count : 1)) launch_m<W, 5, false>(S, cam, set, F, spp0, blocks, st);
-    else launch_m<W, 4, false>(S, cam, set, F, spp0, blocks, st);
+    const uint64_t wave = 6ull * (uint64_t)(sm_count > 0 ? sm_count : 1);
+    if (S.ninst > kLoopPlacements) launch_m<W, 4, 2>(S, cam, set, F, spp0, blocks, st); // the top-level tree
+    else if (S.ninst) launch_m<W, 4, 1>(S, cam, set, F, spp0, blocks, st);
+    // a grid that does not fill the GPU at six blocks per SM gains nothing from more warps: four, no spills
+    else if (blocks < wave) launch_m<W, 4, 0>(S, cam, set, F, spp0, blocks, st);
+    // a few triangles lie in L1 and the kernel is bound by issue: six blocks (80 registers; 12.7 ms on the
+    // box's 36 triangles, 13.9 at eight); more wait on loads: eight (64 registers; 4.63 against 4.67 ms at
+    // 1,602 triangles, 7.06 against 7.41 at 33K, 12.65 against 13.59 at 4.2M)
+    else if (S.ntri < 1024u) launch_m<W, 6, 0>(S, cam, set, F, spp0, blocks, st);
+    else launch_m<W, 8, 0>(S, cam, set, F, spp0, blocks, st);
 }
 
 } // namespace

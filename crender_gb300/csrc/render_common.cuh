@@ -531,6 +531,91 @@ __device__ __forceinline__ bool occluded(const SceneDev &S, v3 o, v3 d, float tm
     return occluded_t<W, CNT, INST>(S, o, d, 1e-5f, tmax, C);
 }
 
+// Closest hit (any = false; tmin 1e-5, world distance below tmax) or any hit
+// (any = true) of one ray per lane, by a whole warp: every lane calls it, `on`
+// says whether the lane has a ray.  The answers are those of closest_t and
+// occluded_t: PL 0 traces a scene of one mesh, 1 its placements by the plain
+// loop, 2 through the top-level tree, one placement per lane at a time.  Any hit:
+// h.prim is a primitive or 0xFFFFFFFF.
+template <int W, bool CNT, int PL>
+__device__ __forceinline__ void warp_trace(const SceneDev &S, WarpRays &sh, bool on, bool any, v3 o, v3 d, float tmax, Hit &h,
+                                           PathCtx &C) {
+    TravStats st{0, 0};
+    LaneTrav T;
+    T.best_prim = 0xFFFFFFFFu;
+    T.best_t = tmax;
+    T.best_slot = 0u;
+    if (PL == 0) {
+        const RayPre r = ray_prep(o.x, o.y, o.z, d.x, d.y, d.z, 1e-5f);
+        warp_traverse<W, CNT>(on, any, r, tmax, 0u, S.nodes, S.tris, sh, T, st, C.err);
+        h.t = T.best_t;
+        h.prim = T.best_prim;
+        h.slot = T.best_slot;
+        h.inst = kNoInst;
+    } else {
+        const bool had = on;
+        TlasRay tr;
+        TlasWalk wk;
+        uint32_t k = 0u; // the lane's placement (the loop's is the same for all lanes)
+        float dl = 1.0f, best = tmax;
+        h.t = 0.0f;
+        h.prim = 0xFFFFFFFFu;
+        h.slot = 0u;
+        h.inst = kNoInst;
+        if (on) {
+            if (PL == 2) {
+                tr = tlas_ray(o, d, 1e-5f);
+                dl = tr.dl;
+                tlas_begin(S, wk);
+                k = tlas_next(S, tr, best, wk);
+            } else {
+                dl = sqrtf(dot(d, d));
+            }
+        }
+        for (;;) {
+            const bool go = on && (PL == 2 ? k != kNoInst : k < S.ninst);
+            if (!__any_sync(0xFFFFFFFFu, go)) break;
+            v3 oo = o, od = d;
+            float bound = 0.0f;
+            uint32_t root = 0u;
+            if (go) {
+                float len;
+                inst_ray(S, k, o, d, oo, od, len);
+                if (any) bound = (tmax * len) / dl;
+                else bound = best < INFINITY ? ((best * len) / dl) * kInstSlack : INFINITY;
+                root = __ldg(&S.inst_root[k]);
+            }
+            const RayPre r = ray_prep(oo.x, oo.y, oo.z, od.x, od.y, od.z, 1e-5f);
+            warp_traverse<W, CNT>(go, any, r, bound, root, S.nodes, S.tris, sh, T, st, C.err);
+            if (go) {
+                if (T.best_prim != 0xFFFFFFFFu) {
+                    if (any) {
+                        h.prim = T.best_prim;
+                        on = false;
+                        continue;
+                    }
+                    const float dist = vdist(inst_point(S, k, oo, od, T.best_t), o);
+                    if (dist < best || (PL == 2 && dist == best && h.inst != kNoInst && k < h.inst)) {
+                        best = dist;
+                        h.t = T.best_t;
+                        h.prim = T.best_prim;
+                        h.slot = T.best_slot;
+                        h.inst = k;
+                    }
+                }
+                if (PL == 2) k = tlas_next(S, tr, best, wk);
+                else ++k;
+            }
+        }
+        if (PL == 2 && had && !wk.ok) C.err = 1u;
+    }
+    h.u = h.v = 0.0f;
+    if (CNT) {
+        C.nodes += st.nodes;
+        C.tris += st.tris;
+    }
+}
+
 // Geometry of a closest hit of the ray (o, d): world point, geometric normal,
 // material index, world distance, and the ray in the triangle's own space (for
 // barycentrics).  WORLD_N = false keeps the object-space normal of an instanced
@@ -994,6 +1079,19 @@ __device__ __forceinline__ bool shadow_visible(const SceneDev &S, const NeeReq &
         if (hit_colour(S, S.mats[hg.mat], sh.prim, sh.slot, hg.ro, hg.rd).w != 0.0f) return false;
         so = add(hg.p, mul(nr.d, 0.1f));
     }
+}
+
+// Pixel at `place` of an image's order of work: 8 x 4 tiles, so that the 32 lanes
+// of a warp start on a compact patch, whose rays share nodes for longer than a
+// row's.  Tiles run along bands of four rows, then come the columns right of the
+// last full tile; a last band of fewer than four rows goes row by row.
+__device__ __forceinline__ uint32_t tile_pixel(uint32_t place, uint32_t w, uint32_t h) {
+    const uint32_t band = place / (4u * w), r = place - band * 4u * w;
+    if (4u * band + 4u > h) return place;
+    const uint32_t tiles = w / 8u, t = r / 32u, k = r % 32u;
+    if (t < tiles) return (4u * band + k / 8u) * w + t * 8u + k % 8u;
+    const uint32_t rest = w - tiles * 8u, q = r - tiles * 32u;
+    return (4u * band + q / rest) * w + tiles * 8u + q % rest;
 }
 
 // camera::get_ray (camera.cpp:14-39)

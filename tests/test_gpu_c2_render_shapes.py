@@ -1,0 +1,26 @@
+"""Megakernel variants by grid and scene size (4, 6 or 8 blocks per SM, pixel tiles
+or rows) against the oracle bit for bit, on images whose sides are no multiples
+of the 8 x 4 tiles."""
+import numpy as np
+import pytest
+
+from crender_gb300 import api, scenes
+from test_gpu_c_render import _assert_identical, _box_variant, _render_both
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("mode,rr", [(1, 3), (0, 0)])
+@pytest.mark.parametrize("size", [(403, 301), (1, 5), (7, 3), (9, 4), (33, 6)])
+def test_small_scene(ctx, orc, size, mode, rr):
+    st = api.make_settings(size[0], size[1], 2, max_bounces=5, rr_depth=rr, mode=mode, seed=71, aspect=size[0] / size[1])
+    kw = dict(sun_enabled=True) if mode == 0 else {}
+    _assert_identical(*_render_both(ctx, orc, _box_variant("materials"), st, passes=2, **kw))
+
+
+@pytest.mark.parametrize("mode,rr", [(1, 3), (0, 0)])
+@pytest.mark.parametrize("size", [(401, 303), (61, 47)])
+def test_larger_scene(ctx, orc, size, mode, rr):
+    sc = scenes.displaced_scene(freq=8)
+    st = api.make_settings(size[0], size[1], 1, max_bounces=8, rr_depth=rr, mode=mode, seed=72, aspect=size[0] / size[1])
+    _assert_identical(*_render_both(ctx, orc, sc, st, skybox=np.ones((1, 1, 4), np.float32)))
