@@ -25,6 +25,8 @@
 // two cancel and nothing is done.  Emitter terms go to a one-entry per-thread
 // cache keyed by the emitter's material.  Gradients accumulate in FP64: per
 // warp in shared memory, then once per block into the caller's arrays.
+#include <type_traits>
+
 #include "render_common.cuh"
 
 namespace crg {
@@ -123,11 +125,17 @@ struct GradTape {
     }
 };
 
-template <int W, bool INST>
-__global__ void __launch_bounds__(128) k_adjoint(SceneDev S, CamDev cam, crg_settings set, const float *__restrict__ adj,
+#ifndef V_AB
+#define V_AB 4
+#endif
+// A warp replays its lanes' paths together, as the forward megakernel traces them.
+template <int W, int PL>
+__global__ void __launch_bounds__(128, V_AB) k_adjoint(SceneDev S, CamDev cam, crg_settings set, const float *__restrict__ adj,
                                                  double *__restrict__ g_col, double *__restrict__ g_em, uint32_t nmat,
                                                  uint32_t copies) {
+    __shared__ WarpRays s_rays[4];
     extern __shared__ double sh[];
+    WarpRays &rays = s_rays[threadIdx.x >> 5];
     double *col = g_col, *em = g_em;
     const uint32_t nacc = 4 * nmat;
     if (copies) {
@@ -137,60 +145,79 @@ __global__ void __launch_bounds__(128) k_adjoint(SceneDev S, CamDev cam, crg_set
         col = mine;
         em = mine + 3 * nmat;
     }
-    const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t place = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t Wd = set.width, Hd = set.height;
+    const bool inside = place < Wd * Hd;
+#ifdef V_ATILE
+    const uint32_t pix = inside ? tile_pixel(place, Wd, Hd) : 0u;
+#else
+    const uint32_t pix = inside ? place : 0u;
+#endif
     PathCtx C{pix, 0, set.seed, 0, 0, 0, 0ull, 0ull};
-    uint32_t lanes = __ballot_sync(0xFFFFFFFFu, pix < Wd * Hd);
-    if (pix < Wd * Hd) {
-        const uint32_t px = pix % Wd, py = pix / Wd;
+    const uint32_t px = pix % Wd, py = pix / Wd;
+    GradTape tape;
+    tape.mats = S.mats;
+    tape.g_col = col;
+    tape.g_em = em;
+    tape.em_mat = 0xffffffffu;
+    tape.dx = tape.dy = tape.dz = 0.0;
+    if (inside) {
         const size_t fidx = (size_t)(Wd - 1 - px) + (size_t)(Hd - 1 - py) * Wd;
         const double inv = 1.0 / (double)set.spp;
-        GradTape tape;
-        tape.mats = S.mats;
-        tape.g_col = col;
-        tape.g_em = em;
-        tape.em_mat = 0xffffffffu;
         tape.dx = (double)adj[fidx * 3] * inv;
         tape.dy = (double)adj[fidx * 3 + 1] * inv;
         tape.dz = (double)adj[fidx * 3 + 2] * inv;
-        const bool live = tape.dx != 0.0 || tape.dy != 0.0 || tape.dz != 0.0;
-        // one loop over segments with path regeneration, as in the forward megakernel
-        PathState ps;
-        Aov aov;
-        uint32_t s = 0, i = 0;
-        for (;;) {
-            // the lanes still replaying meet before every segment (as in the forward megakernel)
-            lanes = __ballot_sync(lanes, live && s < set.spp);
-            if (!(live && s < set.spp)) break;
-            if (i == 0) {
-                C.sample = s;
-                const f4 g0 = rand4(pix, s, 0, set.seed);
-                const float x = ((float)px + g0.x) / (float)Wd;
-                const float y = ((float)py + g0.y) / (float)Hd;
-                v3 o, d;
-                camera_ray(cam, x, y, set.aspect, o, d);
-                path_start(ps, o, d);
-                tape.begin();
-            }
-            if (i < set.max_bounces) {
-                Hit h;
-                const bool found = closest<W, false, INST>(S, ps.o, ps.d, INFINITY, h, C);
-                NeeReq nr;
-                const uint32_t nf = tape.n;
-                const bool cont = shade_extended(S, set, C, i, ps, found, h, aov, nr, &tape);
-                if (nr.kind != 0 && shadow_visible<W, false, INST>(S, nr, C)) {
-                    ps.L = add(ps.L, nr.c);
-                    tape.nee(nr, nf);
-                }
-                ++i;
-                if (cont && i < set.max_bounces) continue;
-            }
-            tape.end();
-            ++s;
-            i = 0;
-        }
-        tape.flush_emitter();
     }
+    tape.begin();
+    const bool live = tape.dx != 0.0 || tape.dy != 0.0 || tape.dz != 0.0;
+    PathState ps;
+    path_start(ps, mk(0, 0, 0), mk(0, 0, 1));
+    // one loop over segments with path regeneration, as in the forward megakernel
+    uint32_t s = live ? 0u : set.spp, i = 0;
+    while (__any_sync(0xFFFFFFFFu, s < set.spp)) {
+        const bool alive = s < set.spp;
+        if (alive && i == 0) {
+            C.sample = s;
+            const f4 g0 = rand4(pix, s, 0, set.seed);
+            const float x = ((float)px + g0.x) / (float)Wd;
+            const float y = ((float)py + g0.y) / (float)Hd;
+            v3 o, d;
+            camera_ray(cam, x, y, set.aspect, o, d);
+            path_start(ps, o, d);
+            tape.begin();
+        }
+        const bool seg = alive && i < set.max_bounces;
+        bool cont = false;
+        NeeReq nr;
+        nr.kind = 0;
+        const uint32_t nf = tape.n;
+#pragma unroll 1
+        for (bool shadow = false;; shadow = true) {
+            const bool on = shadow ? nr.kind != 0 : seg;
+            if (shadow && !__any_sync(0xFFFFFFFFu, on)) break;
+            Hit h;
+            warp_trace<W, false, PL>(S, rays, on, shadow, shadow ? nr.o : ps.o, shadow ? nr.d : ps.d,
+                                     shadow ? nr.tmax : INFINITY, h, C);
+            const bool found = h.prim != 0xFFFFFFFFu;
+            if (!on) continue;
+            if (!shadow) {
+                Aov aov;
+                cont = shade_extended(S, set, C, i, ps, found, h, aov, nr, &tape);
+                continue;
+            }
+            nr.kind = 0;
+            if (!found) {
+                ps.L = add(ps.L, nr.c);
+                tape.nee(nr, nf);
+            }
+        }
+        if (!alive) continue;
+        if (seg && cont && ++i < set.max_bounces) continue;
+        tape.end();
+        ++s;
+        i = 0;
+    }
+    tape.flush_emitter();
     if (C.err) atomicOr(S.err, C.err);
     if (copies) {
         __syncthreads();
@@ -244,23 +271,21 @@ crg_status launch_backward(crg_scene *s, const CamDev &cam, const crg_settings &
     const uint32_t T = 128;
     const uint64_t npix = (uint64_t)set.width * set.height;
     const uint32_t blocks = (uint32_t)((npix + T - 1) / T);
-    // one FP64 accumulator copy per warp when it fits in 48 KB, else one per block, else global atomics
-    const size_t per_copy = sizeof(double) * 4 * (size_t)s->nmat;
-    const uint32_t copies = per_copy * (T / 32) <= 48 * 1024 ? T / 32 : (per_copy <= 48 * 1024 ? 1 : 0);
+    // one FP64 accumulator copy per warp when it fits beside the warps' rays in 48 KB, else one per
+    // block, else global atomics
+    const size_t per_copy = sizeof(double) * 4 * (size_t)s->nmat, room = 48 * 1024 - 4 * sizeof(WarpRays);
+    const uint32_t copies = per_copy * (T / 32) <= room ? T / 32 : (per_copy <= room ? 1 : 0);
     const size_t dyn = per_copy * copies;
+    auto launch = [&](auto width) {
+        constexpr int W = decltype(width)::value;
+        if (S.ninst > kLoopPlacements) k_adjoint<W, 2><<<blocks, T, dyn, st>>>(S, cam, set, adj, g_col, g_em, s->nmat, copies);
+        else if (S.ninst) k_adjoint<W, 1><<<blocks, T, dyn, st>>>(S, cam, set, adj, g_col, g_em, s->nmat, copies);
+        else k_adjoint<W, 0><<<blocks, T, dyn, st>>>(S, cam, set, adj, g_col, g_em, s->nmat, copies);
+    };
     switch (s->width) {
-    case 2:
-        if (S.ninst > kLoopPlacements) k_adjoint<2, true><<<blocks, T, dyn, st>>>(S, cam, set, adj, g_col, g_em, s->nmat, copies);
-        else k_adjoint<2, false><<<blocks, T, dyn, st>>>(S, cam, set, adj, g_col, g_em, s->nmat, copies);
-        break;
-    case 4:
-        if (S.ninst > kLoopPlacements) k_adjoint<4, true><<<blocks, T, dyn, st>>>(S, cam, set, adj, g_col, g_em, s->nmat, copies);
-        else k_adjoint<4, false><<<blocks, T, dyn, st>>>(S, cam, set, adj, g_col, g_em, s->nmat, copies);
-        break;
-    default:
-        if (S.ninst > kLoopPlacements) k_adjoint<8, true><<<blocks, T, dyn, st>>>(S, cam, set, adj, g_col, g_em, s->nmat, copies);
-        else k_adjoint<8, false><<<blocks, T, dyn, st>>>(S, cam, set, adj, g_col, g_em, s->nmat, copies);
-        break;
+    case 2: launch(std::integral_constant<int, 2>{}); break;
+    case 4: launch(std::integral_constant<int, 4>{}); break;
+    default: launch(std::integral_constant<int, 8>{}); break;
     }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_error(s->ctx, e, "k_adjoint launch");

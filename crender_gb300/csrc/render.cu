@@ -1,10 +1,11 @@
-// render.cu — one-thread-per-pixel path-tracing megakernel (sm_103a).
+// render.cu — path-tracing megakernel (sm_103a).
 //
 // The drop-in for cr::renderer's sample passes (CRender
-// src/render/renderer.cpp:116-144, 240-384): each thread owns one pixel,
-// draws settings.spp samples in order and adds them to the pixel's FP32 sum
-// (and optional FP64 sum / sum of squares) in that order, so the film is
-// bit-identical to a sequential CPU accumulation of the same samples.
+// src/render/renderer.cpp:116-144, 240-384): a lane (or one lane of each of a
+// block's four warps) owns a pixel and draws its settings.spp samples, which are
+// added to the pixel's FP32 sum (and optional FP64 sum / sum of squares) in
+// sample order, so the film is bit-identical to a sequential CPU accumulation of
+// the same samples.
 //
 // FAITHFUL follows process_hit / _sample_pixel (renderer.cpp:21-102,
 // 258-384): Lambert = normalize(Ng + uniform sphere point), mirror metal,
@@ -63,22 +64,30 @@ namespace {
 // rows of pixels: box 512x512x64 15.6 -> 12.7 ms (19.6 instead of 11.3 lanes
 // active), 4.2M-triangle mesh 1920x1080x4 15.5 -> 12.7, six placements with the
 // reference estimator 1283x721 1.99 -> 1.23.
-template <int W, int MODE, bool CNT, int MINB, int PL>
+//
+// SPLIT: a block's four warps render the same 32 pixels, a quarter of the samples
+// each, in rounds of kRound samples whose radiances meet in shared memory and
+// are added to the film in sample order; else a warp has its pixels to itself.
+constexpr uint32_t kRound = 64;
+
+template <int W, int MODE, bool CNT, int MINB, int PL, bool SPLIT>
 __global__ void __launch_bounds__(128, MINB) k_render(SceneDev S, CamDev cam, crg_settings set, FilmDev F, uint64_t spp0) {
     __shared__ WarpRays s_rays[4];
-    extern __shared__ double s_sums[]; // films with FP64 planes: 6 sums per thread
+    // SPLIT: the round's radiances [sample][channel][pixel]; else, for films with FP64
+    // planes, 6 sums per thread
+    extern __shared__ double s_sums[];
+    float *s_round = reinterpret_cast<float *>(s_sums);
     WarpRays &sh = s_rays[threadIdx.x >> 5];
-    const uint32_t place = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31u, part = threadIdx.x >> 5;
+    const uint32_t place = SPLIT ? blockIdx.x * 32u + lane : blockIdx.x * 128u + threadIdx.x;
     const uint32_t Wd = set.width, Hd = set.height;
     const bool inside = place < Wd * Hd;
-    // a grid below a wave runs row by row: its time is its slowest block's, and tiles make
-    // blocks less alike (256x256 box forward pass 3% slower with them)
-    const uint32_t pix = inside ? (PL == 0 && MINB == 4 ? place : tile_pixel(place, Wd, Hd)) : 0u;
+    const uint32_t pix = inside ? tile_pixel(place, Wd, Hd) : 0u;
     PathCtx C{pix, 0, set.seed, 0, 0, 0, 0ull, 0ull};
     const uint32_t px = pix % Wd, py = pix / Wd;
-    const size_t fidx = inside ? (size_t)(Wd - 1 - px) + (size_t)(Hd - 1 - py) * Wd : 0;
+    const size_t fidx = (size_t)(Wd - 1 - px) + (size_t)(Hd - 1 - py) * Wd;
     float acc[3] = {0.0f, 0.0f, 0.0f};
-    if (inside) {
+    if (!SPLIT && inside) {
         for (int k = 0; k < 3; ++k) acc[k] = F.sum[fidx * 3 + k];
         if (F.sum64)
             for (int k = 0; k < 3; ++k) {
@@ -88,80 +97,113 @@ __global__ void __launch_bounds__(128, MINB) k_render(SceneDev S, CamDev cam, cr
     }
     PathState ps;
     path_start(ps, mk(0, 0, 0), mk(0, 0, 1));
-    // Path regeneration (Novak, Havran and Dachsbacher 2010): one loop over
-    // segments, in which a lane whose path has ended starts its pixel's next
-    // sample, so a warp runs for the largest total segment count of its lanes
-    // instead of the longest path of every sample.  A pixel's samples still run
-    // and accumulate in order, so the film is unchanged.
-    uint32_t s = inside ? 0u : set.spp, i = 0;
-    while (__any_sync(0xFFFFFFFFu, s < set.spp)) {
-        const bool alive = s < set.spp;
-        if (alive && i == 0) {
-            C.sample = (uint32_t)(spp0 + s);
-            const f4 g0 = rand4(pix, C.sample, 0, set.seed);
-            const float x = ((float)px + g0.x) / (float)Wd;
-            const float y = ((float)py + g0.y) / (float)Hd;
-            v3 o, d;
-            camera_ray(cam, x, y, set.aspect, o, d);
-            path_start(ps, o, d);
-        }
-        const bool seg = alive && i < set.max_bounces;
-        bool cont = false;
-        Aov aov{mk(0, 0, 0), mk(0, 0, 0), 0.0f};
-        NeeReq nr;
-        nr.kind = 0;
-#pragma unroll 1
-        for (bool shadow = false;; shadow = true) {
-            const bool on = shadow ? nr.kind != 0 : seg;
-            if (shadow && !__any_sync(0xFFFFFFFFu, on)) break;
-            Hit h;
-            const v3 o = shadow ? nr.o : ps.o, d = shadow ? nr.d : ps.d;
-            warp_trace<W, CNT, PL>(S, sh, on, shadow && MODE == CRG_MODE_EXTENDED, o, d, shadow ? nr.tmax : INFINITY, h, C);
-            const bool found = h.prim != 0xFFFFFFFFu;
-            if (!on) continue;
-            if (!shadow) {
-                C.segments++;
-                cont = MODE == CRG_MODE_EXTENDED ? shade_extended(S, set, C, i, ps, found, h, aov, nr)
-                                                 : shade_faithful(S, set, C, i, ps, found, h, aov, nr);
-                continue;
+    for (uint32_t base = 0, count = 0; base < set.spp; base += count) {
+        count = SPLIT ? min(kRound, set.spp - base) : set.spp;
+        const uint32_t quarter = (count + 3u) / 4u;
+        // Path regeneration (Novak, Havran and Dachsbacher 2010): one loop over
+        // segments, in which a lane whose path has ended starts its pixel's next
+        // sample, so a warp runs for the largest total segment count of its lanes
+        // instead of the longest path of every sample.  A pixel's samples still
+        // accumulate in order, so the film is unchanged.
+        uint32_t s = base + (SPLIT ? min(count, part * quarter) : 0u), i = 0;
+        const uint32_t end = inside ? (SPLIT ? base + min(count, (part + 1u) * quarter) : set.spp) : s;
+        while (__any_sync(0xFFFFFFFFu, s < end)) {
+            const bool alive = s < end;
+            if (alive && i == 0) {
+                C.sample = (uint32_t)(spp0 + s);
+                const f4 g0 = rand4(pix, C.sample, 0, set.seed);
+                const float x = ((float)px + g0.x) / (float)Wd;
+                const float y = ((float)py + g0.y) / (float)Hd;
+                v3 o, d;
+                camera_ray(cam, x, y, set.aspect, o, d);
+                path_start(ps, o, d);
             }
-            C.shadow++;
+            const bool seg = alive && i < set.max_bounces;
+            bool cont = false;
+            Aov aov{mk(0, 0, 0), mk(0, 0, 0), 0.0f};
+            NeeReq nr;
             nr.kind = 0;
-            if (!found) {
-                ps.L = add(ps.L, nr.c);
-            } else if (MODE == CRG_MODE_FAITHFUL) {
-                // the sun test steps 0.1 past alpha-zero surfaces (renderer.cpp:330-345)
-                const HitGeom hg = hit_geom<false>(S, h, o, d);
-                if (hit_colour(S, S.mats[hg.mat], h.prim, h.slot, hg.ro, hg.rd).w == 0.0f) {
-                    nr.o = add(hg.p, mul(nr.d, 0.1f));
-                    nr.kind = 2;
+#pragma unroll 1
+            for (bool shadow = false;; shadow = true) {
+                const bool on = shadow ? nr.kind != 0 : seg;
+                if (shadow && !__any_sync(0xFFFFFFFFu, on)) break;
+                Hit h;
+                const v3 o = shadow ? nr.o : ps.o, d = shadow ? nr.d : ps.d;
+                warp_trace<W, CNT, PL>(S, sh, on, shadow && MODE == CRG_MODE_EXTENDED, o, d, shadow ? nr.tmax : INFINITY, h, C);
+                const bool found = h.prim != 0xFFFFFFFFu;
+                if (!on) continue;
+                if (!shadow) {
+                    C.segments++;
+                    cont = MODE == CRG_MODE_EXTENDED ? shade_extended(S, set, C, i, ps, found, h, aov, nr)
+                                                     : shade_faithful(S, set, C, i, ps, found, h, aov, nr);
+                    continue;
+                }
+                C.shadow++;
+                nr.kind = 0;
+                if (!found) {
+                    ps.L = add(ps.L, nr.c);
+                } else if (MODE == CRG_MODE_FAITHFUL) {
+                    // the sun test steps 0.1 past alpha-zero surfaces (renderer.cpp:330-345)
+                    const HitGeom hg = hit_geom<false>(S, h, o, d);
+                    if (hit_colour(S, S.mats[hg.mat], h.prim, h.slot, hg.ro, hg.rd).w == 0.0f) {
+                        nr.o = add(hg.p, mul(nr.d, 0.1f));
+                        nr.kind = 2;
+                    }
                 }
             }
+            if (!alive) continue;
+            if (i == 0 && s + 1 == set.spp && F.aov_albedo) { // the last sample's first hit stays
+                reinterpret_cast<float4 *>(F.aov_albedo)[fidx] = make_float4(aov.albedo.x, aov.albedo.y, aov.albedo.z, 1.0f);
+                reinterpret_cast<float4 *>(F.aov_normal)[fidx] =
+                    make_float4(aov.normal.x * 0.5f + 0.5f, aov.normal.y * 0.5f + 0.5f, aov.normal.z * 0.5f + 0.5f, 1.0f);
+                const float dv = mn(aov.depth, 200.0f) / 200.0f;
+                reinterpret_cast<float4 *>(F.aov_depth)[fidx] = make_float4(dv, dv, dv, 1.0f);
+            }
+            if (seg && cont && ++i < set.max_bounces) continue;
+            const v3 L = ps.L;
+            if (SPLIT) {
+                float *q = s_round + (s - base) * 96u + lane;
+                q[0] = L.x;
+                q[32] = L.y;
+                q[64] = L.z;
+            }
+            ++s;
+            i = 0;
+            if (SPLIT) continue;
+            acc[0] += L.x;
+            acc[1] += L.y;
+            acc[2] += L.z;
+            if (F.sum64) {
+                double *q = s_sums + threadIdx.x;
+                q[0] += (double)L.x; q[128] += (double)L.y; q[256] += (double)L.z;
+                q[384] += (double)L.x * (double)L.x;
+                q[512] += (double)L.y * (double)L.y;
+                q[640] += (double)L.z * (double)L.z;
+            }
         }
-        if (!alive) continue;
-        if (i == 0 && s + 1 == set.spp && F.aov_albedo) { // the last sample's first hit stays
-            reinterpret_cast<float4 *>(F.aov_albedo)[fidx] = make_float4(aov.albedo.x, aov.albedo.y, aov.albedo.z, 1.0f);
-            reinterpret_cast<float4 *>(F.aov_normal)[fidx] =
-                make_float4(aov.normal.x * 0.5f + 0.5f, aov.normal.y * 0.5f + 0.5f, aov.normal.z * 0.5f + 0.5f, 1.0f);
-            const float dv = mn(aov.depth, 200.0f) / 200.0f;
-            reinterpret_cast<float4 *>(F.aov_depth)[fidx] = make_float4(dv, dv, dv, 1.0f);
-        }
-        if (seg && cont && ++i < set.max_bounces) continue;
-        ++s;
-        i = 0;
-        const v3 L = ps.L;
-        acc[0] += L.x;
-        acc[1] += L.y;
-        acc[2] += L.z;
-        if (F.sum64) {
-            double *q = s_sums + threadIdx.x;
-            q[0] += (double)L.x; q[128] += (double)L.y; q[256] += (double)L.z;
-            q[384] += (double)L.x * (double)L.x;
-            q[512] += (double)L.y * (double)L.y;
-            q[640] += (double)L.z * (double)L.z;
+        if (SPLIT) {
+            __syncthreads();
+            if (inside && part < 3u) { // warp c adds channel c
+                const size_t k = fidx * 3 + part;
+                const float *q = s_round + part * 32u + lane;
+                float sum = F.sum[k];
+                for (uint32_t j = 0; j < count; ++j) sum += q[j * 96u];
+                F.sum[k] = sum;
+                if (F.sum64) {
+                    double a64 = F.sum64[k], q64 = F.sumsq64[k];
+                    for (uint32_t j = 0; j < count; ++j) {
+                        const double v = (double)q[j * 96u];
+                        a64 += v;
+                        q64 += v * v;
+                    }
+                    F.sum64[k] = a64;
+                    F.sumsq64[k] = q64;
+                }
+            }
+            __syncthreads();
         }
     }
-    if (inside) {
+    if (!SPLIT && inside) {
         for (int k = 0; k < 3; ++k) F.sum[fidx * 3 + k] = acc[k];
         if (F.sum64)
             for (int k = 0; k < 3; ++k) {
@@ -188,35 +230,47 @@ __global__ void __launch_bounds__(128, MINB) k_render(SceneDev S, CamDev cam, cr
     }
 }
 
-template <int W, int MINB, int PL>
-void launch_m(const SceneDev &S, const CamDev &cam, const crg_settings &set, const FilmDev &F, uint64_t spp0,
-              uint32_t blocks, cudaStream_t st) {
-    const uint32_t T = 128;
-    const size_t sums = F.sum64 ? sizeof(double) * 6 * T : 0;
-    if (S.counters) {
-        if (set.mode == CRG_MODE_EXTENDED) k_render<W, CRG_MODE_EXTENDED, true, MINB, PL><<<blocks, T, sums, st>>>(S, cam, set, F, spp0);
-        else k_render<W, CRG_MODE_FAITHFUL, true, MINB, PL><<<blocks, T, sums, st>>>(S, cam, set, F, spp0);
-    } else {
-        if (set.mode == CRG_MODE_EXTENDED) k_render<W, CRG_MODE_EXTENDED, false, MINB, PL><<<blocks, T, sums, st>>>(S, cam, set, F, spp0);
-        else k_render<W, CRG_MODE_FAITHFUL, false, MINB, PL><<<blocks, T, sums, st>>>(S, cam, set, F, spp0);
-    }
+template <int W, int MINB, int PL, bool SPLIT, bool CNT = false>
+void launch_m(const SceneDev &S, const CamDev &cam, const crg_settings &set, const FilmDev &F, uint64_t spp0, cudaStream_t st) {
+    const uint32_t T = 128, per_block = SPLIT ? 32 : T;
+    const uint32_t blocks = (uint32_t)(((uint64_t)set.width * set.height + per_block - 1) / per_block);
+    const size_t shared = SPLIT ? sizeof(float) * 96 * (set.spp < kRound ? set.spp : kRound) : F.sum64 ? sizeof(double) * 6 * T : 0;
+    if (set.mode == CRG_MODE_EXTENDED)
+        k_render<W, CRG_MODE_EXTENDED, CNT, MINB, PL, SPLIT><<<blocks, T, shared, st>>>(S, cam, set, F, spp0);
+    else
+        k_render<W, CRG_MODE_FAITHFUL, CNT, MINB, PL, SPLIT><<<blocks, T, shared, st>>>(S, cam, set, F, spp0);
 }
 
 template <int W>
-void launch_w(const SceneDev &S, const CamDev &cam, const crg_settings &set, const FilmDev &F, uint64_t spp0,
-              int sm_count, cudaStream_t st) {
-    const uint64_t npix = (uint64_t)set.width * set.height;
-    const uint32_t blocks = (uint32_t)((npix + 127) / 128);
-    const uint64_t wave = 6ull * (uint64_t)(sm_count > 0 ? sm_count : 1);
-    if (S.ninst > kLoopPlacements) launch_m<W, 4, 2>(S, cam, set, F, spp0, blocks, st); // the top-level tree
-    else if (S.ninst) launch_m<W, 4, 1>(S, cam, set, F, spp0, blocks, st);
-    // a grid that does not fill the GPU at six blocks per SM gains nothing from more warps: four, no spills
-    else if (blocks < wave) launch_m<W, 4, 0>(S, cam, set, F, spp0, blocks, st);
-    // a few triangles lie in L1 and the kernel is bound by issue: six blocks (80 registers; 12.7 ms on the
-    // box's 36 triangles, 13.9 at eight); more wait on loads: eight (64 registers; 4.63 against 4.67 ms at
-    // 1,602 triangles, 7.06 against 7.41 at 33K, 12.65 against 13.59 at 4.2M)
-    else if (S.ntri < 1024u) launch_m<W, 6, 0>(S, cam, set, F, spp0, blocks, st);
-    else launch_m<W, 8, 0>(S, cam, set, F, spp0, blocks, st);
+void launch_w(const SceneDev &S, const CamDev &cam, const crg_settings &set, const FilmDev &F, uint64_t spp0, int sm_count,
+              cudaStream_t st) {
+    // A few triangles lie in L1 and the kernel is bound by issue: six blocks per SM (80 registers; 12.7 ms
+    // on the box's 36 triangles, 13.9 at eight); more wait on loads: eight (64 registers; 4.63 against 4.67
+    // ms at 1,602 triangles, 7.06 against 7.41 at 33K, 12.65 against 13.59 at 4.2M).
+    const bool small = S.ntri < 1024u;
+    // Splitting a pixel's samples fills the GPU with a quarter of the pixels, evens out the end of the
+    // launch and keeps a tile's rays in one SM's L1: mesh 1920x1080x4 12.8 -> 11.7 ms, 174x136x229 73 ->
+    // 26.8 ms, box 65x70x256 17.1 -> 4.6, 517x333x64 7.1 -> 6.1, 512x512x64 12.8 -> 12.7.  From four
+    // waves of whole warps on a small scene only pays for the rounds: box 1920x1080x16 14.3 -> 15.0.
+    const uint64_t wave = 6ull * (uint64_t)(sm_count > 0 ? sm_count : 1) * 128ull;
+    const bool split = set.spp >= 4 && !(small && !S.ninst && (uint64_t)set.width * set.height >= 4 * wave);
+    if (S.counters) { // the instrumented variants: one form per kind of scene
+        if (S.ninst > kLoopPlacements) launch_m<W, 4, 2, false, true>(S, cam, set, F, spp0, st);
+        else if (S.ninst) launch_m<W, 4, 1, false, true>(S, cam, set, F, spp0, st);
+        else launch_m<W, 4, 0, false, true>(S, cam, set, F, spp0, st);
+    } else if (S.ninst > kLoopPlacements) { // the top-level tree
+        if (split) launch_m<W, 4, 2, true>(S, cam, set, F, spp0, st);
+        else launch_m<W, 4, 2, false>(S, cam, set, F, spp0, st);
+    } else if (S.ninst) {
+        if (split) launch_m<W, 4, 1, true>(S, cam, set, F, spp0, st);
+        else launch_m<W, 4, 1, false>(S, cam, set, F, spp0, st);
+    } else if (small) {
+        if (split) launch_m<W, 6, 0, true>(S, cam, set, F, spp0, st);
+        else launch_m<W, 6, 0, false>(S, cam, set, F, spp0, st);
+    } else {
+        if (split) launch_m<W, 8, 0, true>(S, cam, set, F, spp0, st);
+        else launch_m<W, 8, 0, false>(S, cam, set, F, spp0, st);
+    }
 }
 
 } // namespace

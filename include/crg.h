@@ -523,7 +523,7 @@ crg_status crg_draft_render(crg_scene *scene, const crg_camera *camera, uint32_t
 /* ------------------------------------------------------------------ render */
 
 /* Renders settings->spp more samples per pixel into the film with the
- * one-thread-per-pixel megakernel.  Replaces one or more passes of the
+ * megakernel.  Replaces one or more passes of the
  * renderer's management loop (src/render/renderer.cpp:116-144, 240-384).
  * Sample indices continue from the film's current count, so repeated calls
  * draw fresh, reproducible random numbers. */
