@@ -125,12 +125,17 @@ struct GradTape {
     }
 };
 
-#ifndef V_AB
-#define V_AB 4
-#endif
-// A warp replays its lanes' paths together, as the forward megakernel traces them.
+// A warp replays its lanes' paths together, as the forward megakernel traces
+// them (box 256x256: forward + loss + adjoint of 32 samples 6.39 -> 5.39 ms with
+// it, 4.85 with the samples split as well; 4 blocks of 128 per SM, 3 / 5 / 6
+// measured 6.44 / 5.56 / 5.81).
+//
+// Samples from which they are split over a block's warps: 100x80x32 2.92 -> 1.34
+// ms, 256x256x8 1.48 either way, 384x384x4 1.62 -> 1.76.
+constexpr uint32_t kSplitSpp = 8;
+
 template <int W, int PL>
-__global__ void __launch_bounds__(128, V_AB) k_adjoint(SceneDev S, CamDev cam, crg_settings set, const float *__restrict__ adj,
+__global__ void __launch_bounds__(128, 4) k_adjoint(SceneDev S, CamDev cam, crg_settings set, const float *__restrict__ adj,
                                                  double *__restrict__ g_col, double *__restrict__ g_em, uint32_t nmat,
                                                  uint32_t copies) {
     __shared__ WarpRays s_rays[4];
@@ -145,14 +150,14 @@ __global__ void __launch_bounds__(128, V_AB) k_adjoint(SceneDev S, CamDev cam, c
         col = mine;
         em = mine + 3 * nmat;
     }
-    const uint32_t place = blockIdx.x * blockDim.x + threadIdx.x;
+    // as the forward kernel: 8 x 4 pixel tiles, and with kSplitSpp samples or more a block's warps
+    // replay a quarter of them each for the same 32 pixels
+    const uint32_t parts = set.spp >= kSplitSpp ? 4u : 1u;
+    const uint32_t part = parts == 4u ? threadIdx.x >> 5 : 0u, quarter = (set.spp + parts - 1u) / parts;
+    const uint32_t place = parts == 4u ? blockIdx.x * 32u + (threadIdx.x & 31u) : blockIdx.x * 128u + threadIdx.x;
     const uint32_t Wd = set.width, Hd = set.height;
     const bool inside = place < Wd * Hd;
-#ifdef V_ATILE
     const uint32_t pix = inside ? tile_pixel(place, Wd, Hd) : 0u;
-#else
-    const uint32_t pix = inside ? place : 0u;
-#endif
     PathCtx C{pix, 0, set.seed, 0, 0, 0, 0ull, 0ull};
     const uint32_t px = pix % Wd, py = pix / Wd;
     GradTape tape;
@@ -173,9 +178,10 @@ __global__ void __launch_bounds__(128, V_AB) k_adjoint(SceneDev S, CamDev cam, c
     PathState ps;
     path_start(ps, mk(0, 0, 0), mk(0, 0, 1));
     // one loop over segments with path regeneration, as in the forward megakernel
-    uint32_t s = live ? 0u : set.spp, i = 0;
-    while (__any_sync(0xFFFFFFFFu, s < set.spp)) {
-        const bool alive = s < set.spp;
+    const uint32_t end = min(set.spp, (part + 1u) * quarter);
+    uint32_t s = live ? min(set.spp, part * quarter) : end, i = 0;
+    while (__any_sync(0xFFFFFFFFu, s < end)) {
+        const bool alive = s < end;
         if (alive && i == 0) {
             C.sample = s;
             const f4 g0 = rand4(pix, s, 0, set.seed);
@@ -270,7 +276,8 @@ crg_status launch_backward(crg_scene *s, const CamDev &cam, const crg_settings &
     const SceneDev S = scene_dev(s);
     const uint32_t T = 128;
     const uint64_t npix = (uint64_t)set.width * set.height;
-    const uint32_t blocks = (uint32_t)((npix + T - 1) / T);
+    const uint32_t per_block = set.spp >= kSplitSpp ? T / 4 : T;
+    const uint32_t blocks = (uint32_t)((npix + per_block - 1) / per_block);
     // one FP64 accumulator copy per warp when it fits beside the warps' rays in 48 KB, else one per
     // block, else global atomics
     const size_t per_copy = sizeof(double) * 4 * (size_t)s->nmat, room = 48 * 1024 - 4 * sizeof(WarpRays);

@@ -250,7 +250,8 @@ void launch_w(const SceneDev &S, const CamDev &cam, const crg_settings &set, con
     const bool small = S.ntri < 1024u;
     // Splitting a pixel's samples fills the GPU with a quarter of the pixels, evens out the end of the
     // launch and keeps a tile's rays in one SM's L1: mesh 1920x1080x4 12.8 -> 11.7 ms, 174x136x229 73 ->
-    // 26.8 ms, box 65x70x256 17.1 -> 4.6, 517x333x64 7.1 -> 6.1, 512x512x64 12.8 -> 12.7.  From four
+    // 26.8 ms, box 65x70x256 17.1 -> 4.6, 517x333x64 7.1 -> 6.1, 512x512x64 12.8 -> 12.6
+    // to 14.1 -> 13.8 by camera.  From four
     // waves of whole warps on a small scene only pays for the rounds: box 1920x1080x16 14.3 -> 15.0.
     const uint64_t wave = 6ull * (uint64_t)(sm_count > 0 ? sm_count : 1) * 128ull;
     const bool split = set.spp >= 4 && !(small && !S.ninst && (uint64_t)set.width * set.height >= 4 * wave);

@@ -263,3 +263,26 @@ def test_loss_l2_matches_numpy(ctx):
         for b in (tb, ab, lb):
             b.free()
         P.close()
+
+
+@pytest.mark.parametrize("size,spp", [((1, 1), 1), ((13, 7), 7), ((13, 7), 8), ((13, 7), 9), ((33, 9), 11), ((8, 4), 64)])
+def test_split_replay_matches_oracle(ctx, orc, size, spp):
+    """Replay over partial tiles and with samples split over a block's warps (8 or more)
+    or not.  The oracle adds the same FP64 terms in another order: far below 1e-9."""
+    sc = scenes.inverse_box(np.full((34, 3), 0.5), np.full(3, 0.6))
+    st = api.make_settings(size[0], size[1], spp, max_bounces=6, rr_depth=3, mode=1, seed=81, aspect=size[0] / size[1])
+    adj = np.random.default_rng(82).normal(0, 1, size[0] * size[1] * 3).astype(np.float32)
+    s = api.Scene(ctx, sc["verts"], sc["mat_idx"], sc["mats"]).build()
+    nmat = len(sc["mats"])
+    bufs = [api.DeviceBuffer.from_array(ctx, adj), api.DeviceBuffer.from_array(ctx, np.zeros(3 * nmat)),
+            api.DeviceBuffer.from_array(ctx, np.zeros(nmat))]
+    try:
+        api.backward(s, sc["camera"], st, *bufs)
+        g_col, g_em = bufs[1].download(np.zeros(3 * nmat)), bufs[2].download(np.zeros(nmat))
+    finally:
+        for b in bufs:
+            b.free()
+        s.close()
+    o_col, o_em = orc.adjoint(sc, sc["camera"], st, adj)
+    for a, b in ((g_col, np.asarray(o_col).reshape(-1)), (g_em, np.asarray(o_em).reshape(-1))):
+        assert np.abs(a - b).max() <= 1e-9 * max(np.abs(b).max(), 1e-12)
