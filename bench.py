@@ -834,17 +834,17 @@ def main():
         dst = api.DeviceBuffer(ctx, img.nbytes)
         ps = post_settings_full(api)
         units = W * H
-        # per pixel: pass 0 reads the source and writes 16 B, passes 1-9 read and write 16 B each,
-        # the composite reads source + bloom and writes the output
-        algo = units * (10 * 32 + 48)
+        # per pixel: the threshold reads 16 B and writes 12, four pairs of passes read and write 12 B,
+        # the last pair reads 12 B and the source's 16 and writes the output
+        algo = units * (28 + 4 * 24 + 44)
 
         def step():
             api.post_process(ctx, src, dst, W, H, ps, S)
 
         with ClockSampler(local) as clk:
             ms = timer.steps(step, args.steps, args.warmup)
-        kernel = "k_blur_h / k_blur_v x 10 + k_post_final (one crg_post_process call)"
-        launches = 11 * args.steps
+        kernel = "k_bright + k_bloom x 5 (one crg_post_process call)"
+        launches = 6 * args.steps
         pin_in = api.PinnedArray(ctx, img.shape, np.float32)
         pin_out = api.PinnedArray(ctx, img.shape, np.float32)
         pin_in.array[...] = img

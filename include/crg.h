@@ -503,7 +503,7 @@ crg_status crg_post_settings_default(crg_post_settings *settings);
  * Texels outside the image read as zero.  With no effect enabled the image is
  * copied unchanged, as the reference returns its input.  The blur's two
  * ping-pong images live in a grow-only workspace of the context (2 x W x H x
- * 16 bytes); calls on one context must not overlap. */
+ * 12 bytes, W rounded up to a multiple of 4); calls on one context must not overlap. */
 crg_status crg_post_process(crg_context *ctx, const float *d_src, float *d_dst, uint32_t width, uint32_t height,
                             const crg_post_settings *settings, crg_stream stream);
 

@@ -84,3 +84,14 @@ def test_bad_arguments(ctx):
     assert lib.crg_post_process(ctx.h, b.ptr, c.ptr, 64, 64, s, None) == 1
     b.free()
     c.free()
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("shape", [(1, 1), (7, 27), (8, 28), (15, 29), (31, 113), (33, 8), (40, 64), (1931, 1093)])
+def test_blur_tile_edges_bit_exact(ctx, orc, mode, shape):
+    """Bloom alone (no powf) at the edges of the blur's tiles: widths around 8 and 32,
+    heights around 28 rows and, for the last size, 112."""
+    w, h = shape
+    img = hdr_image(w, h, 91)
+    s = settings(mode=mode, bloom=1, bloom_threshold=0.4, bloom_strength=0.8)
+    assert ulp_diff(run_gpu(ctx, img, s), orc.post_process(img, s)) == 0
