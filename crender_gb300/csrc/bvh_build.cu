@@ -119,16 +119,22 @@ __global__ void k_morton(const float4 *__restrict__ tbox, uint32_t n, const uint
 }
 
 // ----------------------------------------------------------------- radix sort
+// ROWS: keys of a thread; a block sorts 256 ROWS, its warps 32 ROWS consecutive ones
+// each.  Sixteen keep the counts short; two spread a small array over the GPU
+// (a pass over 10,007 keys is the time of one block: 14 us of scatter at 16).
 constexpr int kSortThreads = 256;
-constexpr int kSortTile = 4096; // 8 warps x 512 consecutive keys
+constexpr uint32_t kSmallSort = 1u << 17; // keys up to which ROWS is 2
+constexpr uint32_t sort_blocks(uint32_t n) { return n <= kSmallSort ? (n + 511u) / 512u : (n + 4095u) / 4096u; }
 
+template <int ROWS>
 __global__ void __launch_bounds__(kSortThreads) k_hist(const uint32_t *__restrict__ keys, uint32_t n, int shift,
                                                        uint32_t *__restrict__ hist) {
     __shared__ uint32_t h[256];
     h[threadIdx.x] = 0;
     __syncthreads();
-    const uint32_t base = blockIdx.x * kSortTile;
-    for (int k = 0; k < kSortTile / kSortThreads; ++k) {
+    const uint32_t base = blockIdx.x * (kSortThreads * ROWS);
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) {
         const uint32_t i = base + k * kSortThreads + threadIdx.x;
         if (i < n) atomicAdd(&h[(keys[i] >> shift) & 255u], 1u);
     }
@@ -186,6 +192,7 @@ __global__ void __launch_bounds__(256) k_scan_rows(uint32_t *__restrict__ hist, 
     if (threadIdx.x == 0) digit_sum[blockIdx.x] = run;
 }
 
+template <int ROWS>
 __global__ void __launch_bounds__(kSortThreads) k_scatter(const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin,
                                                           uint32_t n, int shift, const uint32_t *__restrict__ hist,
                                                           const uint32_t *__restrict__ digit_sum,
@@ -202,11 +209,11 @@ __global__ void __launch_bounds__(kSortThreads) k_scatter(const uint32_t *__rest
         goff[tid] = before + hist[tid * gridDim.x + blockIdx.x];
     }
     __syncthreads();
-    const uint32_t base = blockIdx.x * kSortTile + w * 512;
+    const uint32_t base = blockIdx.x * (kSortThreads * ROWS) + w * (32 * ROWS);
     const uint32_t lt = (1u << lane) - 1u;
-    uint32_t kk[16], vv[16], rk[16];
+    uint32_t kk[ROWS], vv[ROWS], rk[ROWS];
 #pragma unroll
-    for (int r = 0; r < 16; ++r) {
+    for (int r = 0; r < ROWS; ++r) {
         const uint32_t i = base + r * 32 + lane;
         const bool valid = i < n;
         const uint32_t key = valid ? kin[i] : 0u;
@@ -233,7 +240,7 @@ __global__ void __launch_bounds__(kSortThreads) k_scatter(const uint32_t *__rest
     }
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < 16; ++r) {
+    for (int r = 0; r < ROWS; ++r) {
         const uint32_t i = base + r * 32 + lane;
         if (i < n) {
             const uint32_t d = (kk[r] >> shift) & 255u;
@@ -904,6 +911,42 @@ __device__ __forceinline__ int floor_log2(double x) {
     return k - 1;
 }
 
+// ceil(log2(ext / 252)) with the quotient rounded to double, for ext > 0, without
+// the division: with ext = m 2^e it is e - 7 for m <= 252/128, else e - 6 (the
+// doubles next to 252 2^k lie further from it than the quotient's rounding can
+// close).  Double arithmetic runs at a sixty-fourth of the float rate here.
+__device__ __forceinline__ int ceil_log2_252nd(double ext) {
+    const uint32_t hi = (uint32_t)__double2hiint(ext), lo = (uint32_t)__double2loint(ext);
+    const uint32_t e = hi >> 20, m = hi & 0xFFFFFu;
+    if (e - 1u >= 0x7FEu) return ceil_log2(ext / 252.0); // infinite, NaN or subnormal
+    return (int)e - 1023 - (m > 0xF8000u || (m == 0xF8000u && lo != 0u) ? 6 : 7);
+}
+
+// Quantized planes of a node's frame: floor((x - p) / 2^e) - 1, at least 0, and
+// ceil((x - p) / 2^e) + 1, at most 255, of the quotient in double, as the CPU form
+// takes them.  x - p is at least a quantum and below 2^9 of them, so its float
+// value decides the whole number unless it is one itself and the exact difference
+// is not; only then is the difference formed in double.
+template <bool HI>
+__device__ __forceinline__ uint32_t quantum_of(float x, float p, float inv_quantum, int e) {
+    const float d = x - p, bb = d - x; // two-sum of x and -p: err is exactly what d dropped
+    const float err = (x - (d - bb)) + (-p - bb);
+    const float q = d * inv_quantum, fl = floorf(q);
+    if (q >= 1.0f && q < 512.0f && (fl != q || err == 0.0f)) {
+        if (HI) return (uint32_t)fminf(ceilf(q) + 1.0f, 255.0f);
+        return (uint32_t)(fl - 1.0f);
+    }
+    const double v = ((double)x - (double)p) * ldexp(1.0, -e);
+    if (HI) {
+        double qh = ceil(v) + 1.0;
+        if (qh > 255.0) qh = 255.0;
+        return (uint32_t)qh;
+    }
+    double ql = floor(v) - 1.0;
+    if (ql < 0.0) ql = 0.0;
+    return (uint32_t)ql;
+}
+
 // Quantizes and writes every node and the triangle slots, eight lanes to a node.
 __global__ void __launch_bounds__(kLevelThreads) k_emit(Collapse C, const LevelState *__restrict__ st) {
     __shared__ __align__(16) uint8_t s_node[kLevelThreads / 8][80];
@@ -934,13 +977,12 @@ __global__ void __launch_bounds__(kLevelThreads) k_emit(Collapse C, const LevelS
             const double ext = hi - lo;
             const double mag = fmax(fabs(lo), fabs(hi));
             int eh = -126;
-            if (ext > 0.0) eh = max(eh, ceil_log2(ext / 252.0));
+            if (ext > 0.0) eh = max(eh, ceil_log2_252nd(ext));
             if (mag > 0.0) eh = max(eh, floor_log2(mag) - 21);
             if (eh > 100) eh = 100;
             ex = eh;
             const double pd = lo - ldexp(1.0, eh);
-            pf = (float)pd;
-            if ((double)pf > pd) pf = nextafterf(pf, -INFINITY);
+            pf = __double2float_rd(pd);
         }
         int e3[3];
         float p3[3];
@@ -975,13 +1017,9 @@ __global__ void __launch_bounds__(kLevelThreads) k_emit(Collapse C, const LevelS
             buf[24 + slot] = (uint8_t)(leafslot ? (((1u << cnt) - 1u) << 5) | toff : 0x20u | (24u + code));
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
-                const double sc = ldexp(1.0, -e3[a]);
-                double ql = floor(((double)b.lo[a] - (double)p3[a]) * sc) - 1.0;
-                double qh = ceil(((double)b.hi[a] - (double)p3[a]) * sc) + 1.0;
-                if (ql < 0.0) ql = 0.0;
-                if (qh > 255.0) qh = 255.0;
-                buf[24 + W + a * W + slot] = (uint8_t)(uint32_t)ql;
-                buf[24 + 4 * W + a * W + slot] = (uint8_t)(uint32_t)qh;
+                const float inv_quantum = __uint_as_float((uint32_t)(127 - e3[a]) << 23);
+                buf[24 + W + a * W + slot] = (uint8_t)quantum_of<false>(b.lo[a], p3[a], inv_quantum, e3[a]);
+                buf[24 + 4 * W + a * W + slot] = (uint8_t)quantum_of<true>(b.hi[a], p3[a], inv_quantum, e3[a]);
             }
         }
         if (c == 0u) {
@@ -1095,7 +1133,7 @@ crg_status build_pipeline(const BvhTarget &t, const crg_build_opts &o, ScratchSo
     if (n == 0) return CRG_OK;
     const uint32_t nint = n >= 2 ? n - 1 : 1;
     const uint32_t node_bytes = ((24 + 7 * o.width) + 15) / 16 * 16;
-    const uint32_t nblk = (n + kSortTile - 1) / kSortTile;
+    const uint32_t nblk = sort_blocks(n);
     auto fail = [&](crg_status s, const std::string &m) {
         if (msg) *msg = m;
         return s;
@@ -1139,9 +1177,11 @@ crg_status build_pipeline(const BvhTarget &t, const crg_build_opts &o, ScratchSo
     {
         uint32_t *ki = k0, *vi = v0, *ko = k1, *vo = v1;
         for (int pass = 0; pass < 4; ++pass) {
-            k_hist<<<nblk, kSortThreads, 0, st>>>(ki, n, pass * 8, hist);
+            if (n <= kSmallSort) k_hist<2><<<nblk, kSortThreads, 0, st>>>(ki, n, pass * 8, hist);
+            else k_hist<16><<<nblk, kSortThreads, 0, st>>>(ki, n, pass * 8, hist);
             k_scan_rows<<<256, 256, 0, st>>>(hist, nblk, digit_sum);
-            k_scatter<<<nblk, kSortThreads, 0, st>>>(ki, vi, n, pass * 8, hist, digit_sum, ko, vo);
+            if (n <= kSmallSort) k_scatter<2><<<nblk, kSortThreads, 0, st>>>(ki, vi, n, pass * 8, hist, digit_sum, ko, vo);
+            else k_scatter<16><<<nblk, kSortThreads, 0, st>>>(ki, vi, n, pass * 8, hist, digit_sum, ko, vo);
             std::swap(ki, ko);
             std::swap(vi, vo);
         }
@@ -1318,7 +1358,7 @@ namespace crg {
 namespace {
 
 constexpr size_t kNaN = CRG_NOALLOC_MAX_TRIS; // max triangles
-constexpr size_t kNaBlk = (kNaN + kSortTile - 1) / kSortTile;
+constexpr size_t kNaBlk = sort_blocks(kNaN);
 constexpr size_t na_round(size_t b) { return (b + 255) / 256 * 256; }
 // the blocks build_pipeline takes for kNaN triangles, each rounded to 256 bytes
 constexpr size_t kNaBytes = 3 * na_round(sizeof(float4) * 2 * kNaN) +    // triangle boxes in both orders, binary nodes
