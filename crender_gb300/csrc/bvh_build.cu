@@ -336,16 +336,24 @@ __device__ __forceinline__ float cost_of_cg(const Tree &T, uint32_t r) {
     return __ldcg(&T.cost[r]);
 }
 
+// Arrival at a node: earlier arrivals.  Releases what the thread (and, after a
+// __syncwarp, its warp) wrote below the node and acquires what the other arrival
+// did: one operation in place of two full fences around a relaxed atomic.
+__device__ __forceinline__ uint32_t arrive(uint32_t *p) {
+    uint32_t old;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(p) : "memory");
+    return old;
+}
+
 // Boxes, primitive counts and SAH costs, the second arrival at a node computing it.
 __global__ void k_bottom_up(Tree T, uint32_t n, uint32_t *__restrict__ visits) {
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
         uint32_t x = T.leaf_parent[j];
         while (x != NONE) {
-            __threadfence();
-            if (atomicAdd(&visits[x], 1u) == 0u) break;
-            __threadfence();
+            // the node's links are there before the arrival and change no more
             const uint32_t up = T.parent[x];
             const uint32_t lc = left_of(T, x), rc = right_of(T, x);
+            if (arrive(&visits[x]) == 0u) break;
             const Box b = merge(box_of_cg(T, lc), box_of_cg(T, rc));
             const float cost = kCi * area(b) + (cost_of_cg(T, lc) + cost_of_cg(T, rc));
             T.count[x] = count_of_cg(T, lc) + count_of_cg(T, rc);
@@ -457,14 +465,14 @@ __device__ __forceinline__ TreeletLeaf treelet_leaf(const Tree &T, uint32_t ref)
 // population count, children read after the choice and one lane rebuilding: two
 // builds of a 4.2M-triangle mesh, one with three rounds, 49.3 -> 21.6 ms; the
 // 10,007-triangle build with three rounds 2.73 -> 1.12 ms.
-__device__ void optimize_treelet(const Tree &T, uint32_t r, TreeletWork &w, const uint8_t *subsets) {
+// `left`, `right` and `root_area` are the root's children and box area.
+__device__ void optimize_treelet(const Tree &T, uint32_t r, uint32_t left, uint32_t right, float root_area, TreeletWork &w,
+                                 const uint8_t *subsets) {
     const uint32_t lane = threadIdx.x & 31u;
-    const TreeletLeaf root = treelet_leaf(T, r);
     TreeletLeaf l{};
     l.ref = LEAF;
-    if (lane < 2u) l = treelet_leaf(T, lane ? root.right : root.left);
-    const float cost_r = kCi * area3(root.hi.x - root.lo.x, root.hi.y - root.lo.y, root.hi.z - root.lo.z) +
-                         (__shfl_sync(0xFFFFFFFFu, l.cost, 0) + __shfl_sync(0xFFFFFFFFu, l.cost, 1));
+    if (lane < 2u) l = treelet_leaf(T, lane ? right : left);
+    const float cost_r = kCi * root_area + (__shfl_sync(0xFFFFFFFFu, l.cost, 0) + __shfl_sync(0xFFFFFFFFu, l.cost, 1));
     int nl = 2;
     while (nl < 7) {
         // the internal leaf of largest area (lowest index on ties); none: the treelet is complete.
@@ -631,26 +639,33 @@ __global__ void __launch_bounds__(128) k_treelet(Tree T, uint32_t n, uint32_t *_
         bool active = x != NONE;
         while (__any_sync(0xFFFFFFFFu, active)) {
             bool need = false;
+            uint32_t up = NONE, left = 0u, right = 0u;
+            float node_area = 0.0f;
             if (active) {
-                __threadfence();
-                if (atomicAdd(&visits[x], 1u) == 0u) {
-                    active = false;
-                } else {
-                    __threadfence();
-                    need = __ldcg(&T.count[x]) >= gamma;
-                }
+                // the node's own record is final (only its parent's treelets will change it), so it is
+                // read while the arrival is under way
+                up = __ldcg(&T.parent[x]);
+                const uint32_t count = __ldcg(&T.count[x]);
+                const float4 lo = __ldcg(&T.nbox[2 * (size_t)x]), hi = __ldcg(&T.nbox[2 * (size_t)x + 1]);
+                left = __float_as_uint(lo.w);
+                right = __float_as_uint(hi.w);
+                node_area = area3(hi.x - lo.x, hi.y - lo.y, hi.z - lo.z);
+                active = arrive(&visits[x]) != 0u;
+                need = active && count >= gamma;
             }
             uint32_t m;
             while ((m = __ballot_sync(0xFFFFFFFFu, need)) != 0u) {
                 const int leader = __ffs(m) - 1;
                 const uint32_t r = __shfl_sync(0xFFFFFFFFu, x, leader);
+                const uint32_t rl = __shfl_sync(0xFFFFFFFFu, left, leader), rr = __shfl_sync(0xFFFFFFFFu, right, leader);
+                const float ra = __shfl_sync(0xFFFFFFFFu, node_area, leader);
                 __syncwarp();
-                optimize_treelet(T, r, s_w[wib], s_subsets);
-                __syncwarp(); // the lanes' writes come before the owner's fence; the working set is free again
+                optimize_treelet(T, r, rl, rr, ra, s_w[wib], s_subsets);
+                __syncwarp(); // the lanes' writes come before the owner's arrival; the working set is free again
                 if ((int)lane == leader) need = false;
             }
             if (active) {
-                x = __ldcg(&T.parent[x]);
+                x = up;
                 if (x == NONE) active = false;
             }
         }
