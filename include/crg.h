@@ -401,7 +401,8 @@ crg_status crg_intersect_closest_counted(const crg_scene *scene, const crg_ray *
 
 /* Traversal schemes of the batched queries (the results are the same):
  *   THREAD: one ray per thread, its group stack in local memory (the default
- *           of crg_intersect_closest / crg_intersect_any);
+ *           of crg_intersect_closest / crg_intersect_any; calls of a few
+ *           thousand rays take WARP's steps, without its refill);
  *   WARP:   W lanes per ray (W = the BVH width), 32 / W rays per warp: the
  *           ray's node is read with 16-byte vector loads by its lanes into
  *           shared memory, each lane tests one child box, pending triangles

@@ -40,3 +40,18 @@ def test_many_block_runs(ctx, orc):
         assert np.array_equal(ga[idx], b.any(np.ascontiguousarray(srays[idx])))
     finally:
         s.close()
+
+
+@pytest.mark.parametrize("width", [8, 4, 2])
+@pytest.mark.parametrize("n", [1, 3, 5, 4095, 4096, 4097, 8192, 8193, 16384, 16385])
+def test_few_rays(ctx, orc, width, n):
+    """Counts around those at which a warp takes one ray, two, four or one per lane."""
+    v = scenes.soup(3000, 47, 0.05)
+    s = api.Scene(ctx, v, np.zeros(len(v), np.uint32), scenes.material_table([{}])).build(width, 1)
+    b = orc.Bvh(v, width=width, treelet=1)
+    try:
+        rays, srays = scenes.soup_rays(n, 48), scenes.soup_rays(n, 49, shadow=True)
+        assert np.array_equal(s.intersect(rays).view(np.uint32), b.closest(rays).view(np.uint32))
+        assert np.array_equal(s.intersect(srays, any_hit=True), b.any(srays))
+    finally:
+        s.close()
