@@ -785,7 +785,7 @@ def main():
             torch.cuda.synchronize()
             work = api.batch_stats(ctx)
             kernel = "wavefront frame: one graph launch"
-            launches = args.steps * (3 + 7 * int(work["iterations"]))
+            launches = args.steps * (2 + 4 * int(work["iterations"]))
         rays = work["segments"] + work["shadow_rays"]
         algo = work["nodes_visited"] * scene.info()["node_bytes"] + work["tris_tested"] * 48 + units * 12
         out["work"] = {**work, "mrays_per_step": rays / 1e6}
@@ -931,10 +931,10 @@ def main():
     value = weak_scaling_value(units, args.steps, world, total_s)
     achieved = algo / (total_s / args.steps) / 1e9
     if launches is None:
-        # per frame: 3 prologue kernels + per device-loop iteration: the bounce kernels (3 split, 2 with the shadow
-        # test in shade, 1 fused) + control, resolve, generate, generated
+        # per frame: 2 prologue kernels + per device-loop iteration: the bounce kernels (3 split, 2 with the shadow
+        # test in shade, 1 fused) + the turn kernel
         fuse = out.get("autotune", {}).get("opts", {}).get("fuse", 1) or 1
-        launches = args.steps * (3 + (4 + (3, 2, 1)[fuse - 1]) * int(out["work"]["iterations"]))
+        launches = args.steps * (2 + (1 + (3, 2, 1)[fuse - 1]) * int(out["work"]["iterations"]))
     traffic, traffic_src = traffic_estimate(args.workload, out, units)
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": traffic, "traffic_source": traffic_src, "kernel": kernel, "peak_kind": peak_kind,

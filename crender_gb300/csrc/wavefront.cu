@@ -10,12 +10,12 @@
 //            to the shadow queue; a finished path writes its sample and the
 //            slot immediately takes the next sample of the batch
 //   shadow   the shadow tests; a visible contribution is added to the path
-//   control  swaps the queues, detects a drained chunk, and sets the graph's
-//            WHILE condition (bounded by an iteration cap that raises
-//            CRG_ERR_TIMEOUT instead of looping forever)
-//   resolve  adds a drained chunk's per-sample radiance to the films in sample
-//            order, so films are bit-identical to the megakernel's
-//   generate seeds the pool with the next chunk's first samples
+//   control  (the last stage's last block) swaps the queues, detects a drained
+//            chunk, and sets the graph's WHILE condition (bounded by an iteration
+//            cap that raises CRG_ERR_TIMEOUT instead of looping forever)
+//   turn     adds a drained chunk's per-sample radiance to the films in sample
+//            order, so films are bit-identical to the megakernel's, and seeds the
+//            pool with the next chunk's first samples
 //
 // A new sample stores only its meta word: extend and shade derive its camera
 // ray, throughput and radiance.  The traversal stages refill idle lanes ray
@@ -67,6 +67,7 @@ struct Ctrl {
     unsigned long long pushed; // entries of the output queue (low 32 bits) and of the shadow queue (high)
     unsigned int in_count;
     unsigned int head_ext, head_shade, head_sh;
+    unsigned int blocks_done;    // of the iteration's last stage
     unsigned int parity;
     unsigned int chunk;          // chunk being rendered
     unsigned int resolve_chunk;  // chunk to resolve this iteration, or ~0u
@@ -207,6 +208,71 @@ __device__ __forceinline__ void finish_and_refill(const Wf &w, Ctrl *c, bool ope
     warp_push(refill, slot, q_out(w, *c), c);
 }
 
+// How the loop's condition is set: in a graph, through its conditional handle.
+struct Loop {
+    cudaGraphConditionalHandle handle;
+    int in_graph;
+};
+
+// Samples that seed the pool for a chunk.
+__device__ __forceinline__ uint32_t seed_count(const Wf &w, const Chunk &ch) {
+    const unsigned long long total = ch.gid_end - ch.gid_begin;
+    return (uint32_t)(total < w.P ? total : w.P);
+}
+
+// Control, by one thread when all other work of the iteration is done: swaps the
+// queues, detects a drained chunk and sets the loop's condition.  What the stage
+// may have changed is read past L1.
+__device__ void wf_control(const Wf &w, Loop loop) {
+    Ctrl *c = w.ctrl;
+    c->blocks_done = 0;
+    if (c->done) { // iterations after the end (host-driven loop) change nothing
+        c->resolve_chunk = 0xFFFFFFFFu;
+        c->generate = 0;
+        if (loop.in_graph) cudaGraphSetConditional(loop.handle, 0u);
+        return;
+    }
+    const unsigned long long pushed = __ldcg(&c->pushed);
+    c->segments += c->in_count;
+    c->shadow += pushed >> 32;
+    c->parity ^= 1u;
+    c->in_count = (unsigned int)pushed;
+    c->pushed = 0;
+    c->head_ext = c->head_shade = c->head_sh = 0;
+    c->resolve_chunk = 0xFFFFFFFFu;
+    c->generate = 0;
+    if (c->in_count == 0) {
+        // chunk drained: resolve it, then seed the next one or stop
+        c->resolve_chunk = c->chunk;
+        if (c->chunk + 1 < w.nchunks) {
+            c->chunk += 1;
+            c->generate = 1;
+            const Chunk ch = w.chunks[c->chunk];
+            c->in_count = seed_count(w, ch);
+            c->issued = ch.gid_begin + c->in_count;
+        } else {
+            c->done = 1;
+        }
+    }
+    c->iterations += 1;
+    if (c->iterations >= c->max_iterations && !c->done) {
+        c->error = __ldcg(&c->error) | 2u; // bounded loop ran out
+        c->done = 1;
+    }
+    if (loop.in_graph) cudaGraphSetConditional(loop.handle, c->done ? 0u : 1u);
+}
+
+// The end of an iteration's last stage: the block that finishes last runs the
+// control step (a kernel of its own cost its launch in every iteration).
+__device__ __forceinline__ void end_iteration(const Wf &w, Loop loop) {
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(&w.ctrl->blocks_done, 1u) + 1u != gridDim.x) return;
+    __threadfence();
+    wf_control(w, loop);
+}
+
 template <int W, bool CNT, bool INST>
 __global__ void __launch_bounds__(256) k_wf_extend(Wf w) {
     unsigned long long nodes = 0, tris = 0;
@@ -255,7 +321,7 @@ __global__ void __launch_bounds__(256) k_wf_extend(Wf w) {
 // Contributions reach L in the same order in every form: emission of bounce
 // i, its NEE, then bounce i + 1.
 template <int W, int FUSE, bool CNT, bool INST>
-__global__ void __launch_bounds__(256, FUSE == 0 ? 3 : 2) k_wf_shade(Wf w) {
+__global__ void __launch_bounds__(256, FUSE == 0 ? 3 : 2) k_wf_shade(Wf w, Loop loop) {
     unsigned long long nodes = 0, tris = 0;
     Ctrl *c = w.ctrl;
     const unsigned int n = c->in_count;
@@ -371,10 +437,11 @@ __global__ void __launch_bounds__(256, FUSE == 0 ? 3 : 2) k_wf_shade(Wf w) {
         atomicAdd(FUSE == 1 ? &c->nodes_sh : &c->nodes, nodes);
         atomicAdd(FUSE == 1 ? &c->tris_sh : &c->tris, tris);
     }
+    if (FUSE >= 1) end_iteration(w, loop);
 }
 
 template <int W, bool CNT, bool INST>
-__global__ void __launch_bounds__(256) k_wf_shadow(Wf w) {
+__global__ void __launch_bounds__(256) k_wf_shadow(Wf w, Loop loop) {
     unsigned long long nodes = 0, tris = 0;
     Ctrl *c = w.ctrl;
     const unsigned int n = sh_count(c);
@@ -424,6 +491,7 @@ __global__ void __launch_bounds__(256) k_wf_shadow(Wf w) {
         atomicAdd(&c->nodes_sh, nodes);
         atomicAdd(&c->tris_sh, tris);
     }
+    end_iteration(w, loop);
 }
 
 // Lanes without pending triangles below which a warp of the traversal stages
@@ -553,7 +621,7 @@ __global__ void __launch_bounds__(256, 4) k_wf_extend_dyn(Wf w) {
 // (occluded_placement_loop, occluded_placements), stopping at the first
 // placement that occludes.
 template <int W, bool CNT, int PL>
-__global__ void __launch_bounds__(256, 4) k_wf_shadow_dyn(Wf w) {
+__global__ void __launch_bounds__(256, 4) k_wf_shadow_dyn(Wf w, Loop loop) {
     Ctrl *c = w.ctrl;
     const unsigned int n = sh_count(c);
     const bool open = samples_open(w, c);
@@ -640,47 +708,11 @@ __global__ void __launch_bounds__(256, 4) k_wf_shadow_dyn(Wf w) {
         atomicAdd(&c->nodes_sh, (unsigned long long)st.nodes);
         atomicAdd(&c->tris_sh, (unsigned long long)st.tris);
     }
+    end_iteration(w, loop);
 }
 
-__global__ void k_wf_control(Wf w, cudaGraphConditionalHandle handle, int in_graph) {
-    if (threadIdx.x != 0) return;
-    Ctrl *c = w.ctrl;
-    if (c->done) { // iterations after the end (host-driven loop) change nothing
-        c->resolve_chunk = 0xFFFFFFFFu;
-        c->generate = 0;
-        if (in_graph) cudaGraphSetConditional(handle, 0u);
-        return;
-    }
-    c->segments += c->in_count;
-    c->shadow += sh_count(c);
-    c->parity ^= 1u;
-    c->in_count = (unsigned int)c->pushed;
-    c->pushed = 0;
-    c->head_ext = c->head_shade = c->head_sh = 0;
-    c->resolve_chunk = 0xFFFFFFFFu;
-    c->generate = 0;
-    if (c->in_count == 0) {
-        // chunk drained: resolve it, then seed the next one or stop
-        c->resolve_chunk = c->chunk;
-        if (c->chunk + 1 < w.nchunks) {
-            c->chunk += 1;
-            c->generate = 1;
-        } else {
-            c->done = 1;
-        }
-    }
-    c->iterations += 1;
-    if (c->iterations >= c->max_iterations && !c->done) {
-        c->error |= 2u; // bounded loop ran out
-        c->done = 1;
-    }
-    if (in_graph) cudaGraphSetConditional(handle, c->done ? 0u : 1u);
-}
-
-__global__ void k_wf_resolve(Wf w) {
-    const Ctrl *c = w.ctrl;
-    const uint32_t k = c->resolve_chunk;
-    if (k == 0xFFFFFFFFu) return;
+// Adds chunk k's per-sample radiance to the films, in sample order.
+__device__ void wf_resolve(const Wf &w, uint32_t k) {
     const Chunk ch = w.chunks[k];
     for (uint32_t item = blockIdx.x * blockDim.x + threadIdx.x; item < ch.resolve_items; item += gridDim.x * blockDim.x) {
         uint32_t lo = ch.seg_begin, hi = ch.seg_end - 1;
@@ -727,13 +759,14 @@ __global__ void k_wf_resolve(Wf w) {
     }
 }
 
-// Seeds the pool with the first min(P, chunk size) samples of the chunk.
-__global__ void k_wf_generate(Wf w, int first) {
-    Ctrl *c = w.ctrl;
-    if (!first && !c->generate) return;
+// Between iterations: resolves a drained chunk and seeds the pool with the next
+// one's first min(P, chunk size) samples (the two touch different memory).
+__global__ void k_wf_turn(Wf w) {
+    const Ctrl *c = w.ctrl;
+    if (c->resolve_chunk != 0xFFFFFFFFu) wf_resolve(w, c->resolve_chunk);
+    if (!c->generate) return;
     const Chunk ch = w.chunks[c->chunk];
-    const unsigned long long total = ch.gid_end - ch.gid_begin;
-    const uint32_t count = (uint32_t)(total < w.P ? total : w.P);
+    const uint32_t count = seed_count(w, ch);
     uint32_t *in = q_in(w, *c);
     for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < count; slot += gridDim.x * blockDim.x) {
         start_sample(w, slot, ch.gid_begin + slot, ch);
@@ -741,25 +774,16 @@ __global__ void k_wf_generate(Wf w, int first) {
     }
 }
 
-// Sets the counts after a generate (one thread; runs after k_wf_generate).
-__global__ void k_wf_generated(Wf w, int first) {
-    if (threadIdx.x != 0) return;
-    Ctrl *c = w.ctrl;
-    if (!first && !c->generate) return;
-    const Chunk ch = w.chunks[c->chunk];
-    const unsigned long long total = ch.gid_end - ch.gid_begin;
-    const uint32_t count = (uint32_t)(total < w.P ? total : w.P);
-    c->in_count = count;
-    c->issued = ch.gid_begin + count;
-    c->generate = 0;
-}
-
-__global__ void k_wf_start(Ctrl *c, unsigned int max_iterations) {
+// The control block before the first iteration: chunk 0 to be seeded.
+__global__ void k_wf_start(Wf w, unsigned int max_iterations) {
     if (threadIdx.x != 0) return;
     Ctrl z{};
     z.resolve_chunk = 0xFFFFFFFFu;
     z.max_iterations = max_iterations;
-    *c = z;
+    z.generate = 1;
+    z.in_count = seed_count(w, w.chunks[0]);
+    z.issued = w.chunks[0].gid_begin + z.in_count;
+    *w.ctrl = z;
 }
 
 struct Workspace {
@@ -819,23 +843,23 @@ void launch_extend_dyn(const Wf &wf, uint32_t grid, uint32_t block, cudaStream_t
     else k_wf_extend_dyn<W, CNT, 0><<<grid, block, dyn_shared(block), st>>>(wf);
 }
 template <int W, bool CNT, bool INST>
-void launch_shadow_dyn(const Wf &wf, uint32_t grid, uint32_t block, cudaStream_t st) {
-    if (INST) k_wf_shadow_dyn<W, CNT, 2><<<grid, block, dyn_shared(block), st>>>(wf);
-    else if (wf.placed) k_wf_shadow_dyn<W, CNT, 1><<<grid, block, dyn_shared(block), st>>>(wf);
-    else k_wf_shadow_dyn<W, CNT, 0><<<grid, block, dyn_shared(block), st>>>(wf);
+void launch_shadow_dyn(const Wf &wf, Loop loop, uint32_t grid, uint32_t block, cudaStream_t st) {
+    if (INST) k_wf_shadow_dyn<W, CNT, 2><<<grid, block, dyn_shared(block), st>>>(wf, loop);
+    else if (wf.placed) k_wf_shadow_dyn<W, CNT, 1><<<grid, block, dyn_shared(block), st>>>(wf, loop);
+    else k_wf_shadow_dyn<W, CNT, 0><<<grid, block, dyn_shared(block), st>>>(wf, loop);
 }
 
 // The per-bounce kernels of one loop iteration for a fusion level.
 template <int W, int FUSE, bool CNT, bool INST>
-void launch_bounce(const Wf &wf, const Grids &g, uint32_t block, cudaStream_t st) {
+void launch_bounce(const Wf &wf, Loop loop, const Grids &g, uint32_t block, cudaStream_t st) {
     if (FUSE <= 1) {
         if (wf.refill) launch_extend_dyn<W, CNT, INST>(wf, g.ext, block, st);
         else k_wf_extend<W, CNT, INST><<<g.ext, block, 0, st>>>(wf);
     }
-    k_wf_shade<W, FUSE, CNT, INST><<<g.shade, block, 0, st>>>(wf);
+    k_wf_shade<W, FUSE, CNT, INST><<<g.shade, block, 0, st>>>(wf, loop);
     if (FUSE == 0) {
-        if (wf.refill_sh) launch_shadow_dyn<W, CNT, INST>(wf, g.shadow, block, st);
-        else k_wf_shadow<W, CNT, INST><<<g.shadow, block, 0, st>>>(wf);
+        if (wf.refill_sh) launch_shadow_dyn<W, CNT, INST>(wf, loop, g.shadow, block, st);
+        else k_wf_shadow<W, CNT, INST><<<g.shadow, block, 0, st>>>(wf, loop);
     }
 }
 
@@ -843,8 +867,8 @@ void launch_bounce(const Wf &wf, const Grids &g, uint32_t block, cudaStream_t st
 // done flag every 8 iterations (for profilers that cannot see into graphs
 // with conditional nodes, and for runtimes without them).  With `times`, CUDA
 // events on the stream bracket every stage of every iteration and the device
-// time of each stage is summed into it: extend, shade, shadow, and the
-// control / resolve / generate kernels.
+// time of each stage is summed into it: extend, shade, shadow (with the control
+// step), and the turn kernel.
 template <int W, int FUSE, bool CNT, bool INST>
 crg_status run_host(crg_context *ctx, const Wf &wf, uint32_t grid, const Grids &bg, uint32_t block, uint32_t max_iters,
                     cudaStream_t st, crg_stage_times *times) {
@@ -864,6 +888,7 @@ crg_status run_host(crg_context *ctx, const Wf &wf, uint32_t grid, const Grids &
     auto mark = [&](uint32_t it, int m) {
         if (times) cudaEventRecord(ev[(it % kWin) * kMarks + m], st);
     };
+    const Loop loop{0, 0};
     for (uint32_t it = 0; rc == CRG_OK && it < max_iters + 8; ++it) {
         mark(it, 0);
         if (FUSE <= 1) {
@@ -871,17 +896,14 @@ crg_status run_host(crg_context *ctx, const Wf &wf, uint32_t grid, const Grids &
             else k_wf_extend<W, CNT, INST><<<bg.ext, block, 0, st>>>(wf);
         }
         mark(it, 1);
-        k_wf_shade<W, FUSE, CNT, INST><<<bg.shade, block, 0, st>>>(wf);
+        k_wf_shade<W, FUSE, CNT, INST><<<bg.shade, block, 0, st>>>(wf, loop);
         mark(it, 2);
         if (FUSE == 0) {
-            if (wf.refill_sh) launch_shadow_dyn<W, CNT, INST>(wf, bg.shadow, block, st);
-            else k_wf_shadow<W, CNT, INST><<<bg.shadow, block, 0, st>>>(wf);
+            if (wf.refill_sh) launch_shadow_dyn<W, CNT, INST>(wf, loop, bg.shadow, block, st);
+            else k_wf_shadow<W, CNT, INST><<<bg.shadow, block, 0, st>>>(wf, loop);
         }
         mark(it, 3);
-        k_wf_control<<<1, 32, 0, st>>>(wf, 0, 0);
-        k_wf_resolve<<<grid, 256, 0, st>>>(wf);
-        k_wf_generate<<<grid, 256, 0, st>>>(wf, 0);
-        k_wf_generated<<<1, 32, 0, st>>>(wf, 0);
+        k_wf_turn<<<grid, 256, 0, st>>>(wf);
         mark(it, 4);
         if ((it % kWin) == kWin - 1) {
             cudaError_t e = cudaMemcpyAsync(done_h, &wf.ctrl->done, sizeof(unsigned int), cudaMemcpyDeviceToHost, st);
@@ -990,7 +1012,7 @@ crg_status cached_graph(crg_context *ctx, const Wf &wf, const Grids &bg, uint32_
         cudaGraphDestroy(g.graph);
         B->graphs.erase(B->graphs.begin() + (long)lru);
     }
-    // one graph: WHILE (not done) { extend, shade, shadow, control, resolve, generate }
+    // one graph: WHILE (not done) { extend, shade, shadow (its last block: control), turn }
     GraphEntry e;
     e.key = key;
     cudaStream_t cap = nullptr;
@@ -1021,11 +1043,8 @@ crg_status cached_graph(crg_context *ctx, const Wf &wf, const Grids &bg, uint32_
             rc = cuda_error(ctx, er, "cudaStreamBeginCaptureToGraph");
             break;
         }
-        launch_bounce<W, FUSE, CNT, INST>(wf, bg, block, cap);
-        k_wf_control<<<1, 32, 0, cap>>>(wf, handle, 1);
-        k_wf_resolve<<<grid, 256, 0, cap>>>(wf);
-        k_wf_generate<<<grid, 256, 0, cap>>>(wf, 0);
-        k_wf_generated<<<1, 32, 0, cap>>>(wf, 0);
+        launch_bounce<W, FUSE, CNT, INST>(wf, Loop{handle, 1}, bg, block, cap);
+        k_wf_turn<<<grid, 256, 0, cap>>>(wf);
         er = cudaStreamEndCapture(cap, &body);
         if (er != cudaSuccess) { rc = cuda_error(ctx, er, "cudaStreamEndCapture"); break; }
         if ((er = cudaGraphInstantiate(&e.exec, e.graph, 0)) != cudaSuccess) {
@@ -1053,9 +1072,8 @@ template <int W, int FUSE, bool CNT, bool INST>
 crg_status run(crg_context *ctx, const Wf &wf, uint32_t grid, uint32_t block, uint32_t max_iters, cudaStream_t st,
                uint32_t host_loop) {
     // prologue on the caller's stream
-    k_wf_start<<<1, 32, 0, st>>>(wf.ctrl, max_iters);
-    k_wf_generate<<<grid, 256, 0, st>>>(wf, 1);
-    k_wf_generated<<<1, 32, 0, st>>>(wf, 1);
+    k_wf_start<<<1, 32, 0, st>>>(wf, max_iters);
+    k_wf_turn<<<grid, 256, 0, st>>>(wf);
     CRG_CUDA(ctx, cudaGetLastError());
     Grids bg{0, 0, 0};
     {
