@@ -1388,7 +1388,8 @@ crg_status batch_call(crg_scene *const *scenes, uint32_t nscenes, const crg_view
     // defaults: up to 128M paths in flight (about 20 GB of path state for a batch that large; a
     // frame never holds more paths than its largest chunk's samples), 128M-sample chunks (2 GB of
     // sample slots), split stages with per-lane refill in the traversal stages
-    crg_wavefront_opts o{1u << 27, 1u << 27, 128, 32, 0, 0, 0, 1, 16};
+    // (fuse 0: render_batch takes 1, or 3 for a small pool)
+    crg_wavefront_opts o{1u << 27, 1u << 27, 128, 32, 0, 0, 0, 0, 16};
     if (opts) {
         if (opts->path_pool) o.path_pool = opts->path_pool;
         if (opts->chunk_samples) o.chunk_samples = opts->chunk_samples;
@@ -1398,6 +1399,7 @@ crg_status batch_call(crg_scene *const *scenes, uint32_t nscenes, const crg_view
         o.count_work = opts->count_work;
         o.host_loop = opts->host_loop;
         if (opts->fuse) o.fuse = opts->fuse;
+        else if (opts->block_size || opts->fetch || opts->refill) o.fuse = 1; // options of the split stages
         if (opts->refill) o.refill = opts->refill == 0xFFFFFFFFu ? 0u : opts->refill;
     }
     if ((o.block_size != 64 && o.block_size != 128 && o.block_size != 256) || o.fetch % 32 || o.fetch > 4096 ||

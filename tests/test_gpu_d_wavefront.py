@@ -395,3 +395,19 @@ def test_queue_edges_match_megakernel(ctx, size, spp, opts):
         f.close()
     finally:
         s.close()
+
+
+@pytest.mark.parametrize("samples", [1 << 19, (1 << 19) + 1024])
+def test_default_fusion_by_pool(ctx, samples):
+    """The default form on either side of the pool size from which stages are split."""
+    sc = _box_variant("materials")
+    s = api.Scene(ctx, sc["verts"], sc["mat_idx"], sc["mats"]).build()
+    st = api.make_settings(1024, samples // 1024, 1, max_bounces=4, rr_depth=0, mode=1, seed=33)
+    try:
+        ref = _mega(ctx, s, sc["camera"], st)
+        f = api.Film(ctx, st.width, st.height, f64=True)
+        ctx.check(api.render_batch([s], [(0, sc["camera"], st)], [f]))
+        _same(f.download(f64=True), ref)
+        f.close()
+    finally:
+        s.close()
