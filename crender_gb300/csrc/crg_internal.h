@@ -91,7 +91,7 @@ struct crg_scene {
     uint32_t nlights = 0;
     std::vector<double> tri_area; // per-triangle area (host), for rebuilding the emitter table
     DevBuf light_prim, light_alias, light_pdf, mat_light_pdf; // light_alias: float2 {prob, alias bits}
-    DevBuf light_rec; // float4[4] per emitter entry: world corners, pdf, prim, material, radiance
+    DevBuf light_rec; // float4[5] per emitter entry: world corners, pdf, prim, material, radiance, normal
     // environment / sun
     DevBuf sky;
     uint32_t sky_w = 0, sky_h = 0;

@@ -293,12 +293,14 @@ __global__ void k_light_records(SceneDev S, float4 *__restrict__ rec) {
     }
     const uint32_t mi = S.mat_idx[prim];
     const crg_material &m = S.mats[mi];
-    float4 *r = rec + 4 * (size_t)j;
+    float4 *r = rec + kLightVec * (size_t)j;
     r[0] = make_float4(a.x, a.y, a.z, S.light_pdf[j]);
     r[1] = make_float4(b.x, b.y, b.z, __uint_as_float(prim));
     r[2] = make_float4(c.x, c.y, c.z, __uint_as_float(mi));
     r[3] = make_float4(m.colour[0] * m.emission, m.colour[1] * m.emission, m.colour[2] * m.emission,
                        __uint_as_float(textured(S, m) ? 1u : 0u));
+    const v3 n = normalize(cross(sub(b, a), sub(c, a)));
+    r[4] = make_float4(n.x, n.y, n.z, 0.0f);
 }
 
 } // namespace
@@ -307,7 +309,7 @@ __global__ void k_light_records(SceneDev S, float4 *__restrict__ rec) {
 // table, the materials, the textures or the instances change).
 crg_status build_light_records(crg_scene *s) {
     if (s->nlights == 0) return CRG_OK;
-    crg_status rc = dev_alloc(s->ctx, s->light_rec, 64 * (size_t)s->nlights);
+    crg_status rc = dev_alloc(s->ctx, s->light_rec, sizeof(float4) * kLightVec * (size_t)s->nlights);
     if (rc != CRG_OK) return rc;
     const SceneDev S = scene_dev(s);
     k_light_records<<<(s->nlights + 127) / 128, 128>>>(S, (float4 *)s->light_rec.ptr);

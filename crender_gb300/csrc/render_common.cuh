@@ -40,8 +40,8 @@ struct SceneDev {
     const float4 *tlas;         // top-level tree over the placements (4 float4 per node)
     uint32_t tlas_root;         // its root: a node index, or kTlasLeaf | placement
     const uint32_t *light_inst; // instance of each emitter entry (instanced scenes)
-    // per emitter entry 4 float4: (v0, pdf), (v1, prim bits), (v2, material bits), (colour * emission,
-    // textured flag bits); v0..v2 in world space
+    // per emitter entry 5 float4: (v0, pdf), (v1, prim bits), (v2, material bits), (colour * emission,
+    // textured flag bits), (geometric normal, -); v0..v2 and the normal in world space
     const float4 *light_rec;
     uint32_t ninst;
     uint32_t nlights, ntri;
@@ -58,6 +58,8 @@ struct SceneDev {
 
 // Device view of a built scene (defined in render.cu).
 SceneDev scene_dev(const crg_scene *s);
+
+constexpr uint32_t kLightVec = 5; // float4 per emitter record
 
 struct FilmDev {
     float *sum;
@@ -878,8 +880,8 @@ __device__ inline void nee_prepare(const SceneDev &S, const PathCtx &C, uint32_t
     const f4 g = rand4(C.pix, C.sample, 2 + 2 * i, C.seed);
     const uint32_t j = pick_light(S, g.x, g.w);
     // the emitter entry's record: world-space corners, pdf, primitive, material, radiance
-    const float4 r0 = __ldg(&S.light_rec[4 * (size_t)j + 0]), r1 = __ldg(&S.light_rec[4 * (size_t)j + 1]);
-    const float4 r2 = __ldg(&S.light_rec[4 * (size_t)j + 2]), r3 = __ldg(&S.light_rec[4 * (size_t)j + 3]);
+    const float4 *rec = S.light_rec + kLightVec * (size_t)j;
+    const float4 r0 = __ldg(rec), r1 = __ldg(rec + 1), r2 = __ldg(rec + 2), r3 = __ldg(rec + 3), r4 = __ldg(rec + 4);
     const v3 a = mk(r0.x, r0.y, r0.z), b = mk(r1.x, r1.y, r1.z), c = mk(r2.x, r2.y, r2.z);
     const uint32_t prim = __float_as_uint(r1.w), lmi = __float_as_uint(r2.w);
     const float su = sqrtf(g.y);
@@ -893,8 +895,7 @@ __device__ inline void nee_prepare(const SceneDev &S, const PathCtx &C, uint32_t
     const v3 wi = mul(w, 1.0f / dist);
     const float cos_s = dot(wi, n);
     if (!(cos_s > 0.0f)) return;
-    const v3 Ngl = normalize(cross(sub(b, a), sub(c, a)));
-    const float cos_l = absf(dot(Ngl, wi));
+    const float cos_l = absf(dot(mk(r4.x, r4.y, r4.z), wi));
     if (!(cos_l > 0.0f)) return;
     v3 Le = mk(r3.x, r3.y, r3.z); // colour * emission
     if (__float_as_uint(r3.w)) {   // textured emitter: texture colour at the sampled point * emission

@@ -173,11 +173,12 @@ __device__ void start_sample(const Wf &w, uint32_t slot, unsigned long long gid,
     }
     const Segment sg = w.segs[lo];
     const ViewDev &V = w.views[sg.view];
-    const unsigned long long rel = gid - sg.gid;
-    const uint32_t s = sg.s0 + (uint32_t)(rel / V.npix);
-    const uint32_t pix = (uint32_t)(rel % V.npix);
-    const uint32_t sample = (uint32_t)(V.spp0 + s);
-    w.meta[slot] = make_uint4(sg.view | kPrevDelta | kFresh, pix, sample, (uint32_t)(gid - ch.gid_begin));
+    // a segment lies in its chunk, whose samples are counted in 32 bits
+    const uint32_t rel = (uint32_t)(gid - sg.gid), row = rel / V.npix, place = rel - row * V.npix;
+    const uint32_t pix = tile_pixel(place, V.set.width, V.set.height);
+    const uint32_t sample = (uint32_t)(V.spp0 + sg.s0 + row);
+    // issued tile by tile; the radiance's place is the pixel's, as the film is resolved row by row
+    w.meta[slot] = make_uint4(sg.view | kPrevDelta | kFresh, pix, sample, (uint32_t)(gid - ch.gid_begin) - place + pix);
 }
 
 // Whether the chunk may have samples left to issue (read when a stage starts).
