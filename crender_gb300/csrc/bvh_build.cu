@@ -397,21 +397,40 @@ __device__ const SubsetTable kSubsets = make_subsets();
 template <int K> constexpr int kSubsetFirst = K == 2 ? 0 : K == 3 ? 21 : K == 4 ? 56 : K == 5 ? 91 : 112;
 
 // Costs of the subsets of size K: one lane per subset, its 2^(K-1) - 1
-// partitions (those with the lowest leaf) in the CPU form's order.
+// partitions (those with the lowest leaf) in the CPU form's order.  A
+// partition's cells follow from an earlier one's by an addition each: part j
+// without its highest leaf's cell is a part already formed, and the other half
+// is what is left of the whole.
 template <int K>
 __device__ __forceinline__ void treelet_subsets(TreeletWork &w, const uint8_t *subsets, int nsub, uint32_t lane) {
     for (int i = kSubsetFirst<K> + (int)lane; i < kSubsetFirst<K + 1>; i += 32) {
         const int s = subsets[i];
         if (s >= nsub) continue;
-        const int low = s & -s, rest = s ^ low;
-        float best = FLT_MAX;
-        int bp = 0, q = rest;
+        // part[j]: the lowest leaf and those of the others but the highest that j's bits choose
+        constexpr int H = 1 << (K - 2);
+        int part[H];
+        int left = s & (s - 1);
+        part[0] = s ^ left;
 #pragma unroll
-        for (int t = 0; t < (1 << (K - 1)) - 1; ++t) {
-            q = (q - 1) & rest;
-            const int P = q | low;
-            const float c = w.cS[P] + w.cS[s ^ P];
+        for (int k = 0; k < K - 2; ++k) {
+            const int bit = left & -left;
+            left ^= bit;
+#pragma unroll
+            for (int j = 0; j < (1 << k); ++j) part[j + (1 << k)] = part[j] + bit;
+        }
+        // the parts with the highest leaf (`left` by now), the whole set apart, and then those without
+        float best = FLT_MAX;
+        int bp = part[0];
+#pragma unroll
+        for (int j = H - 2; j >= 0; --j) {
+            const int P = part[j] + left;
+            const float c = w.cS[P] + w.cS[s - P];
             if (c < best) { best = c; bp = P; }
+        }
+#pragma unroll
+        for (int j = H - 1; j >= 0; --j) {
+            const float c = w.cS[part[j]] + w.cS[s - part[j]];
+            if (c < best) { best = c; bp = part[j]; }
         }
         w.cS[s] = kCi * w.aS[s] + best;
         w.pS[s] = (uint8_t)bp;
@@ -426,23 +445,23 @@ struct TreeletLeaf {
     float cost;
 };
 __device__ __forceinline__ TreeletLeaf treelet_leaf(const Tree &T, uint32_t ref) {
+    // leaves and nodes by the same loads: the two lanes that read at a time do not wait for one another
+    const bool leaf = (ref & LEAF) != 0u;
+    const size_t j = ref & ~LEAF;
+    const float4 *p = leaf ? T.lbox : T.nbox;
     TreeletLeaf l;
     l.ref = ref;
-    if (ref & LEAF) {
-        const size_t j = ref & ~LEAF;
-        l.lo = T.lbox[2 * j];
-        l.hi = T.lbox[2 * j + 1];
-        l.left = l.right = 0u;
-        l.count = 1u;
-        l.cost = kCt * area3(l.hi.x - l.lo.x, l.hi.y - l.lo.y, l.hi.z - l.lo.z);
-    } else {
-        l.lo = __ldcg(&T.nbox[2 * (size_t)ref]);
-        l.hi = __ldcg(&T.nbox[2 * (size_t)ref + 1]);
-        l.left = __float_as_uint(l.lo.w);
-        l.right = __float_as_uint(l.hi.w);
-        l.count = __ldcg(&T.count[ref]);
-        l.cost = __ldcg(&T.cost[ref]);
+    l.lo = __ldcg(&p[2 * j]);
+    l.hi = __ldcg(&p[2 * j + 1]);
+    l.count = 1u;
+    float cost = 0.0f;
+    if (!leaf) {
+        l.count = __ldcg(&T.count[j]);
+        cost = __ldcg(&T.cost[j]);
     }
+    l.left = __float_as_uint(l.lo.w);
+    l.right = __float_as_uint(l.hi.w);
+    l.cost = leaf ? kCt * area3(l.hi.x - l.lo.x, l.hi.y - l.lo.y, l.hi.z - l.lo.z) : cost;
     return l;
 }
 
@@ -621,53 +640,57 @@ __device__ void optimize_treelet(const Tree &T, uint32_t r, uint32_t left, uint3
     }
 }
 
-// Bottom-up pass over the tree by warps of 32 leaves: a lane goes on to a
-// node's parent only on the node's second arrival (both subtrees final); the
-// nodes of at least `gamma` leaves that the lanes reach in a step are
-// restructured one after another by the whole warp.  Launched with 128
-// threads per block.
-__global__ void __launch_bounds__(128) k_treelet(Tree T, uint32_t n, uint32_t *__restrict__ visits, uint32_t gamma) {
-    __shared__ TreeletWork s_w[4];
+// Bottom-up pass over the tree, a warp starting from `per` leaves: a lane goes
+// on to a node's parent only on the node's second arrival (both subtrees final);
+// the nodes of at least `gamma` leaves that the lanes reach in a step are
+// restructured one after another by the whole warp.
+//
+// A block is one warp, so that its place is free as soon as its climb ends
+// (climbs differ in length by the tree's depth), and 64 registers let the 32
+// blocks of an SM run at once: with the subsets' cells by one addition and leaves
+// and nodes read by the same loads, two builds of a 4.2M-triangle mesh, one with
+// three rounds, 11.7 -> 10.6 ms (blocks of two warps 10.7, of four 11.1; left at
+// 89 registers 11.9).
+__global__ void __launch_bounds__(32, 32) k_treelet(Tree T, uint32_t n, uint32_t *__restrict__ visits, uint32_t gamma,
+                                                    uint32_t per) {
+    __shared__ TreeletWork s_w;
     __shared__ uint8_t s_subsets[112];
-    const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
-    if (threadIdx.x < 112u) s_subsets[threadIdx.x] = kSubsets.s[threadIdx.x];
-    __syncthreads();
-    const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
-    for (uint32_t base = (blockIdx.x * (blockDim.x >> 5) + wib) * 32u; base < n; base += nwarps * 32u) {
-        const uint32_t j = base + lane;
-        uint32_t x = j < n ? __ldcg(&T.leaf_parent[j]) : NONE;
-        bool active = x != NONE;
-        while (__any_sync(0xFFFFFFFFu, active)) {
-            bool need = false;
-            uint32_t up = NONE, left = 0u, right = 0u;
-            float node_area = 0.0f;
-            if (active) {
-                // the node's own record is final (only its parent's treelets will change it), so it is
-                // read while the arrival is under way
-                up = __ldcg(&T.parent[x]);
-                const uint32_t count = __ldcg(&T.count[x]);
-                const float4 lo = __ldcg(&T.nbox[2 * (size_t)x]), hi = __ldcg(&T.nbox[2 * (size_t)x + 1]);
-                left = __float_as_uint(lo.w);
-                right = __float_as_uint(hi.w);
-                node_area = area3(hi.x - lo.x, hi.y - lo.y, hi.z - lo.z);
-                active = arrive(&visits[x]) != 0u;
-                need = active && count >= gamma;
-            }
-            uint32_t m;
-            while ((m = __ballot_sync(0xFFFFFFFFu, need)) != 0u) {
-                const int leader = __ffs(m) - 1;
-                const uint32_t r = __shfl_sync(0xFFFFFFFFu, x, leader);
-                const uint32_t rl = __shfl_sync(0xFFFFFFFFu, left, leader), rr = __shfl_sync(0xFFFFFFFFu, right, leader);
-                const float ra = __shfl_sync(0xFFFFFFFFu, node_area, leader);
-                __syncwarp();
-                optimize_treelet(T, r, rl, rr, ra, s_w[wib], s_subsets);
-                __syncwarp(); // the lanes' writes come before the owner's arrival; the working set is free again
-                if ((int)lane == leader) need = false;
-            }
-            if (active) {
-                x = up;
-                if (x == NONE) active = false;
-            }
+    const uint32_t lane = threadIdx.x;
+    for (uint32_t i = lane; i < 112u; i += 32u) s_subsets[i] = kSubsets.s[i];
+    __syncwarp();
+    const uint32_t j = blockIdx.x * per + lane;
+    uint32_t x = lane < per && j < n ? __ldcg(&T.leaf_parent[j]) : NONE;
+    bool active = x != NONE;
+    while (__any_sync(0xFFFFFFFFu, active)) {
+        bool need = false;
+        uint32_t up = NONE, left = 0u, right = 0u;
+        float node_area = 0.0f;
+        if (active) {
+            // the node's own record is final (only its parent's treelets will change it), so it is
+            // read while the arrival is under way
+            up = __ldcg(&T.parent[x]);
+            const uint32_t count = __ldcg(&T.count[x]);
+            const float4 lo = __ldcg(&T.nbox[2 * (size_t)x]), hi = __ldcg(&T.nbox[2 * (size_t)x + 1]);
+            left = __float_as_uint(lo.w);
+            right = __float_as_uint(hi.w);
+            node_area = area3(hi.x - lo.x, hi.y - lo.y, hi.z - lo.z);
+            active = arrive(&visits[x]) != 0u;
+            need = active && count >= gamma;
+        }
+        uint32_t m;
+        while ((m = __ballot_sync(0xFFFFFFFFu, need)) != 0u) {
+            const int leader = __ffs(m) - 1;
+            const uint32_t r = __shfl_sync(0xFFFFFFFFu, x, leader);
+            const uint32_t rl = __shfl_sync(0xFFFFFFFFu, left, leader), rr = __shfl_sync(0xFFFFFFFFu, right, leader);
+            const float ra = __shfl_sync(0xFFFFFFFFu, node_area, leader);
+            __syncwarp();
+            optimize_treelet(T, r, rl, rr, ra, s_w, s_subsets);
+            __syncwarp(); // the lanes' writes come before the owner's arrival; the working set is free again
+            if ((int)lane == leader) need = false;
+        }
+        if (active) {
+            x = up;
+            if (x == NONE) active = false;
         }
     }
 }
@@ -1208,10 +1231,16 @@ crg_status build_pipeline(const BvhTarget &t, const crg_build_opts &o, ScratchSo
         BP_CHECK(cudaMemsetAsync(visits, 0, sizeof(uint32_t) * nint, st));
         k_bottom_up<<<grid_for(n, T), T, 0, st>>>(Tr, n, visits);
         if (o.treelet) {
-            uint32_t gamma = 7;
+            // a warp takes 32 leaves where that still makes as many warps as run at once, and down to two
+            // where it does not: its treelets wait for one another, those of different warps do not.
+            // Three rounds over 10,007 triangles and the rest of the build 574 us with 32 leaves, 540 with
+            // 8, 511 with 2, 517 with 1; 33,282 triangles, two builds, 1.355 ms with 32, 1.300 with 4;
+            // 163,282 triangles 1.71 ms with 32, 1.72 with 16, 1.76 with 8.
+            uint32_t gamma = 7, per = 32;
+            while (per > 2u && n / per < 152u * 32u) per /= 2u;
             for (uint32_t round = 0; round < o.treelet_rounds; ++round) {
                 BP_CHECK(cudaMemsetAsync(visits, 0, sizeof(uint32_t) * nint, st));
-                k_treelet<<<grid_for(n, 128), 128, 0, st>>>(Tr, n, visits, gamma);
+                k_treelet<<<(n + per - 1) / per, 32, 0, st>>>(Tr, n, visits, gamma, per);
                 gamma *= 2;
             }
             // every node's cost is its children's and its area's still: a node of at least gamma leaves

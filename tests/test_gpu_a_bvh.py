@@ -88,3 +88,19 @@ def test_treelet_edges_bit_exact(ctx, orc, n, rounds):
     assert gi == o.info()
     for a, b in zip(g, o.download()):
         assert np.array_equal(a.view(np.uint8), b.view(np.uint8))
+
+
+@pytest.mark.parametrize("n", [9727, 9728, 19457, 38912, 77825, 155649])
+def test_treelet_leaves_per_warp_bit_exact(ctx, orc, n):
+    """Either side of the sizes at which a warp of the treelet kernel takes twice
+    as many leaves (2 to 32 of them), the last block only partly filled."""
+    v = np.ascontiguousarray(scenes.soup(n, 90, 0.05))
+    s = api.Scene(ctx, v, np.zeros(n, np.uint32), _mats()).build(8, 1, 3, 2)
+    try:
+        gi, g = s.info(), s.download_bvh()
+    finally:
+        s.close()
+    o = orc.Bvh(v, width=8, treelet=1, leaf_max=3, rounds=2)
+    assert gi == o.info()
+    for a, b in zip(g, o.download()):
+        assert np.array_equal(a.view(np.uint8), b.view(np.uint8))
