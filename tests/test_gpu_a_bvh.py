@@ -104,3 +104,23 @@ def test_treelet_leaves_per_warp_bit_exact(ctx, orc, n):
     assert gi == o.info()
     for a, b in zip(g, o.download()):
         assert np.array_equal(a.view(np.uint8), b.view(np.uint8))
+
+
+@pytest.mark.parametrize("same", [0, 1])
+@pytest.mark.parametrize("n", [2, 127, 128, 129, 256, 385, 1025])
+def test_climb_edges_bit_exact(ctx, orc, n, same):
+    """Trees at the edges of the bottom-up pass's blocks of 128 leaves, of scattered
+    triangles and of many at one place (equal codes: the tree follows the indices)."""
+    v = np.ascontiguousarray(scenes.soup(n, 70 + n, 0.1))
+    if same:
+        v[:] = v[:1]
+        v[n // 2:, 0] += np.float32(1e-4)
+    s = api.Scene(ctx, v, np.zeros(n, np.uint32), _mats()).build(8, 0, 1)
+    try:
+        gi, g = s.info(), s.download_bvh()
+    finally:
+        s.close()
+    o = orc.Bvh(v, width=8, treelet=0, leaf_max=1)
+    assert gi == o.info()
+    for a, b in zip(g, o.download()):
+        assert np.array_equal(a.view(np.uint8), b.view(np.uint8))
