@@ -70,16 +70,24 @@ namespace {
 // are added to the film in sample order; else a warp has its pixels to itself.
 constexpr uint32_t kRound = 64;
 
+// A warp with its pixels to itself is a block, whose place is free again as soon as
+// the warp ends: box 1920x1080x8 7.36 -> 6.88 ms against blocks of four, mesh
+// 1920x1080x1 3.23 -> 3.16.  Not with placements, where neighbouring warps do better
+// close together (six placements 1283x721x1 1.24, 1.30 so).
+template <int PL, bool SPLIT> constexpr uint32_t kRenderThreads = SPLIT || PL ? 128 : 32;
+
 template <int W, int MODE, bool CNT, int MINB, int PL, bool SPLIT>
-__global__ void __launch_bounds__(128, MINB) k_render(SceneDev S, CamDev cam, crg_settings set, FilmDev F, uint64_t spp0) {
-    __shared__ WarpRays s_rays[4];
+__global__ void __launch_bounds__((kRenderThreads<PL, SPLIT>), MINB * 128 / kRenderThreads<PL, SPLIT>)
+k_render(SceneDev S, CamDev cam, crg_settings set, FilmDev F, uint64_t spp0) {
+    constexpr uint32_t T = kRenderThreads<PL, SPLIT>;
+    __shared__ WarpRays s_rays[T / 32];
     // SPLIT: the round's radiances [sample][channel][pixel]; else, for films with FP64
     // planes, 6 sums per thread
     extern __shared__ double s_sums[];
     float *s_round = reinterpret_cast<float *>(s_sums);
     WarpRays &sh = s_rays[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u, part = threadIdx.x >> 5;
-    const uint32_t place = SPLIT ? blockIdx.x * 32u + lane : blockIdx.x * 128u + threadIdx.x;
+    const uint32_t place = SPLIT ? blockIdx.x * 32u + lane : blockIdx.x * T + threadIdx.x;
     const uint32_t Wd = set.width, Hd = set.height;
     const bool inside = place < Wd * Hd;
     const uint32_t pix = inside ? tile_pixel(place, Wd, Hd) : 0u;
@@ -91,8 +99,8 @@ __global__ void __launch_bounds__(128, MINB) k_render(SceneDev S, CamDev cam, cr
         for (int k = 0; k < 3; ++k) acc[k] = F.sum[fidx * 3 + k];
         if (F.sum64)
             for (int k = 0; k < 3; ++k) {
-                s_sums[k * 128 + threadIdx.x] = F.sum64[fidx * 3 + k];
-                s_sums[(3 + k) * 128 + threadIdx.x] = F.sumsq64[fidx * 3 + k];
+                s_sums[k * T + threadIdx.x] = F.sum64[fidx * 3 + k];
+                s_sums[(3 + k) * T + threadIdx.x] = F.sumsq64[fidx * 3 + k];
             }
     }
     PathState ps;
@@ -175,10 +183,10 @@ __global__ void __launch_bounds__(128, MINB) k_render(SceneDev S, CamDev cam, cr
             acc[2] += L.z;
             if (F.sum64) {
                 double *q = s_sums + threadIdx.x;
-                q[0] += (double)L.x; q[128] += (double)L.y; q[256] += (double)L.z;
-                q[384] += (double)L.x * (double)L.x;
-                q[512] += (double)L.y * (double)L.y;
-                q[640] += (double)L.z * (double)L.z;
+                q[0] += (double)L.x; q[T] += (double)L.y; q[2 * T] += (double)L.z;
+                q[3 * T] += (double)L.x * (double)L.x;
+                q[4 * T] += (double)L.y * (double)L.y;
+                q[5 * T] += (double)L.z * (double)L.z;
             }
         }
         if (SPLIT) {
@@ -207,8 +215,8 @@ __global__ void __launch_bounds__(128, MINB) k_render(SceneDev S, CamDev cam, cr
         for (int k = 0; k < 3; ++k) F.sum[fidx * 3 + k] = acc[k];
         if (F.sum64)
             for (int k = 0; k < 3; ++k) {
-                F.sum64[fidx * 3 + k] = s_sums[k * 128 + threadIdx.x];
-                F.sumsq64[fidx * 3 + k] = s_sums[(3 + k) * 128 + threadIdx.x];
+                F.sum64[fidx * 3 + k] = s_sums[k * T + threadIdx.x];
+                F.sumsq64[fidx * 3 + k] = s_sums[(3 + k) * T + threadIdx.x];
             }
     }
     if (C.err) atomicOr(S.err, C.err);
@@ -232,7 +240,8 @@ __global__ void __launch_bounds__(128, MINB) k_render(SceneDev S, CamDev cam, cr
 
 template <int W, int MINB, int PL, bool SPLIT, bool CNT = false>
 void launch_m(const SceneDev &S, const CamDev &cam, const crg_settings &set, const FilmDev &F, uint64_t spp0, cudaStream_t st) {
-    const uint32_t T = 128, per_block = SPLIT ? 32 : T;
+    constexpr uint32_t T = kRenderThreads<PL, SPLIT>;
+    const uint32_t per_block = SPLIT ? 32 : T;
     const uint32_t blocks = (uint32_t)(((uint64_t)set.width * set.height + per_block - 1) / per_block);
     const size_t shared = SPLIT ? sizeof(float) * 96 * (set.spp < kRound ? set.spp : kRound) : F.sum64 ? sizeof(double) * 6 * T : 0;
     if (set.mode == CRG_MODE_EXTENDED)
@@ -249,10 +258,10 @@ void launch_w(const SceneDev &S, const CamDev &cam, const crg_settings &set, con
     // ms at 1,602 triangles, 7.06 against 7.41 at 33K, 12.65 against 13.59 at 4.2M).
     const bool small = S.ntri < 1024u;
     // Splitting a pixel's samples fills the GPU with a quarter of the pixels, evens out the end of the
-    // launch and keeps a tile's rays in one SM's L1: mesh 1920x1080x4 12.8 -> 11.7 ms, 174x136x229 73 ->
-    // 26.8 ms, box 65x70x256 17.1 -> 4.6, 517x333x64 7.1 -> 6.1, 512x512x64 12.8 -> 12.6
-    // to 14.1 -> 13.8 by camera.  From four
-    // waves of whole warps on a small scene only pays for the rounds: box 1920x1080x16 14.3 -> 15.0.
+    // launch and keeps a tile's rays in one SM's L1: mesh 1920x1080x4 12.4 -> 11.6 ms, 174x136x229 98 ->
+    // 35, box 65x70x256 14.7 -> 4.6, 517x333x64 6.3 -> 5.9.  A view of a small scene that fills the GPU
+    // four times only pays for the rounds (box 800x600x16 4.45 -> 4.59, 1920x1080x16 13.1 -> 14.7); from
+    // twice on it goes either way by the view (512x512x64 11.8 -> 12.4, 700x500x64 13.3 -> 12.6).
     const uint64_t wave = 6ull * (uint64_t)(sm_count > 0 ? sm_count : 1) * 128ull;
     const bool split = set.spp >= 4 && !(small && !S.ninst && (uint64_t)set.width * set.height >= 4 * wave);
     if (S.counters) { // the instrumented variants: one form per kind of scene
