@@ -115,10 +115,10 @@ def measured_peaks():
 POST = dict(width=3840, height=2160)
 # leaf sizes the autotuner tries per scene (bit mask of 1 << leaf_max)
 LEAVES = (1 << 1) | (1 << 2) | (1 << 3)
-# (width, treelet, leaf_max) fastest for the megakernel in a GB300 sweep of width {4, 8} x leaf {1, 2, 3}
-# x treelet rounds {3, 6}: box 616-623 Msamples/s at width 4 (592 at 8), displaced 655 at width 4 leaf 1
-# (579 at width 8 leaf 3)
-MEGA_BVH = {"box": (4, 1, 2), "displaced": (4, 1, 1)}
+# (width, treelet, leaf_max) fastest for the megakernel in a GB300 sweep of width {2, 4, 8} x leaf {1, 2, 3}:
+# box 512x512x64 1,230 Msamples/s at width 8 leaf 3 (991 at width 4, 760 at 2), displaced 1920x1080x16 927 at
+# width 4 leaf 3 (912 at width 8 leaf 3, 850 / 842 at leaf 1)
+MEGA_BVH = {"box": (8, 1, 3), "displaced": (4, 1, 3)}
 
 
 def post_settings_full(api):
@@ -751,8 +751,7 @@ def main():
         else:
             sc = scenes.displaced_scene()
             st = api.make_settings(1920, 1080, 16, 16, 3, 1, 1, 1920 / 1080)
-        # the megakernel on its own best BVH; the wavefront form on width 8 with the leaf size its tuner
-        # picks for each scene (box 3, displaced 1)
+        # the megakernel on its own best BVH; the wavefront form on width 8
         bvh = MEGA_BVH[args.workload] if args.form == "megakernel" else (8, 1, 3 if args.workload == "box" else 1)
         scene = api.Scene(ctx, sc["verts"], sc["mat_idx"], sc["mats"]).build(*bvh)
         out["bvh"] = dict(zip(("width", "treelet", "leaf_max"), bvh))
@@ -894,7 +893,7 @@ def main():
         occluded = int(ob.download(np.zeros(n, np.uint32)).astype(bool).sum())
         out["any_hit"] = {"value": n / (sum(ms_any) / len(ms_any) / 1e3) / 1e6, "unit": "Mrays/s",
                           "ms_per_step": sum(ms_any) / len(ms_any), "rays": n, "occluded_fraction": occluded / n,
-                          "kernel": "k_intersect_dyn<8> (any hit, per-lane refill)"}
+                          "kernel": "k_intersect<8, any> (any hit, per-lane refill)"}
         # the warp-cooperative scheme on the same rays (8 lanes per ray, nodes staged in shared memory)
         ms_wc = timer.steps(lambda: ctx.check(lib.crg_intersect_closest_with(scene.h, rb.ptr, hb.ptr, n,
                                                                              api.TRAVERSAL_WARP, S)),
