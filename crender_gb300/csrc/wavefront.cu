@@ -227,7 +227,7 @@ __device__ __forceinline__ uint32_t seed_count(const Wf &w, const Chunk &ch) {
 __device__ void wf_control(const Wf &w, Loop loop) {
     Ctrl *c = w.ctrl;
     c->blocks_done = 0;
-    if (c->done) { // iterations after the end (host-driven loop) change nothing
+    if (c->done) { // iterations after the end (host-driven loop) find empty queues and change nothing
         c->resolve_chunk = 0xFFFFFFFFu;
         c->generate = 0;
         if (loop.in_graph) cudaGraphSetConditional(loop.handle, 0u);
@@ -259,6 +259,8 @@ __device__ void wf_control(const Wf &w, Loop loop) {
     if (c->iterations >= c->max_iterations && !c->done) {
         c->error = __ldcg(&c->error) | 2u; // bounded loop ran out
         c->done = 1;
+        c->in_count = 0; // what is still queued is given up: no later stage may take it up again
+        c->generate = 0;
     }
     if (loop.in_graph) cudaGraphSetConditional(loop.handle, c->done ? 0u : 1u);
 }
