@@ -215,11 +215,11 @@ template <int W> __device__ __forceinline__ uint32_t nbyte(const uint32_t *w, in
     return (w[b >> 2] >> ((b & 3) * 8)) & 0xFFu;
 }
 
-// Bytes k and k + 1 of `word` as exact floats 2^15 + q: one PRMT each (q is the
-// second byte of the float's bits).
+// Bytes k and k + 1 of `word` as exact floats 1/2 + q 2^-16: one PRMT each (q is
+// the second byte of the float's bits).
 __device__ __forceinline__ float2 qbias(uint32_t word, int k) {
-    return make_float2(__uint_as_float(__byte_perm(word, 0x47000000u, 0x7604u | (uint32_t)k << 4)),
-                       __uint_as_float(__byte_perm(word, 0x47000000u, 0x7604u | (uint32_t)(k + 1) << 4)));
+    return make_float2(__uint_as_float(__byte_perm(word, 0x3F000000u, 0x7604u | (uint32_t)k << 4)),
+                       __uint_as_float(__byte_perm(word, 0x3F000000u, 0x7604u | (uint32_t)(k + 1) << 4)));
 }
 
 // Every byte of x filled with its top bit.
@@ -287,9 +287,11 @@ __device__ __forceinline__ void visit_node(const uint4 *__restrict__ nodes, uint
     }
     const float px = __uint_as_float(w[0]), py = __uint_as_float(w[1]), pz = __uint_as_float(w[2]);
     const uint32_t eb = w[3];
-    const float sx = __uint_as_float((eb & 0xFFu) << 23) * r.ix;
-    const float sy = __uint_as_float(((eb >> 8) & 0xFFu) << 23) * r.iy;
-    const float sz = __uint_as_float(((eb >> 16) & 0xFFu) << 23) * r.iz;
+    // widths 8 and 4 take a quantum times 2^16 (exponent bytes are at most 227: no carry)
+    const uint32_t es = W == 2 ? eb : eb + 0x00101010u;
+    const float sx = __uint_as_float((es & 0xFFu) << 23) * r.ix;
+    const float sy = __uint_as_float(((es >> 8) & 0xFFu) << 23) * r.iy;
+    const float sz = __uint_as_float(((es >> 16) & 0xFFu) << 23) * r.iz;
     const float ox = (px - r.ox) * r.ix;
     const float oy = (py - r.oy) * r.iy;
     const float oz = (pz - r.oz) * r.iz;
@@ -301,9 +303,13 @@ __device__ __forceinline__ void visit_node(const uint4 *__restrict__ nodes, uint
         constexpr int LO = (24 + W) / 4, HI = (24 + 4 * W) / 4, ME = 24 / 4;
         const bool nxs = r.ix < 0.0f, nys = r.iy < 0.0f, nzs = r.iz < 0.0f;
         const float2 sx2 = make_float2(sx, sx), sy2 = make_float2(sy, sy), sz2 = make_float2(sz, sz);
-        // the plane parameters are formed from 2^15 + q, so the offset takes 2^15 quanta off:
-        // that rounds to within 2^-9 quantum, and the boxes hold a whole quantum of slack per side
-        const float bx = __fmaf_rn(-32768.0f, sx, ox), by = __fmaf_rn(-32768.0f, sy, oy), bz = __fmaf_rn(-32768.0f, sz, oz);
+        // the plane parameters are formed from 1/2 + q 2^-16, so the offset takes 2^15 quanta off:
+        // that rounds to within 2^-9 quantum, and the boxes hold a whole quantum of slack per side.
+        // On an axis the ray hardly moves along, 2^16 quanta may be infinite (from a quantum of 2^32
+        // with a zero direction): both planes are then infinity less infinity, a NaN that the minima
+        // and maxima pass over, so the axis is left out of the test.  Where 2^16 quanta are finite,
+        // an infinite offset is one of planes beyond 2^126, on the side where they lie.
+        const float bx = __fmaf_rn(-0.5f, sx, ox), by = __fmaf_rn(-0.5f, sy, oy), bz = __fmaf_rn(-0.5f, sz, oz);
         const float2 ox2 = make_float2(bx, bx), oy2 = make_float2(by, by), oz2 = make_float2(bz, bz);
         const uint32_t oct4 = oct * 0x01010101u;
 #pragma unroll
