@@ -12,6 +12,7 @@
 
 #include "crg_dev.cuh"
 #include "crg_internal.h"
+#include "work_order.h"
 
 namespace crg {
 namespace rc {
@@ -1080,19 +1081,6 @@ __device__ __forceinline__ bool shadow_visible(const SceneDev &S, const NeeReq &
         if (hit_colour(S, S.mats[hg.mat], sh.prim, sh.slot, hg.ro, hg.rd).w != 0.0f) return false;
         so = add(hg.p, mul(nr.d, 0.1f));
     }
-}
-
-// Pixel at `place` of an image's order of work: 8 x 4 tiles, so that the 32 lanes
-// of a warp start on a compact patch, whose rays share nodes for longer than a
-// row's.  Tiles run along bands of four rows, then come the columns right of the
-// last full tile; a last band of fewer than four rows goes row by row.
-__device__ __forceinline__ uint32_t tile_pixel(uint32_t place, uint32_t w, uint32_t h) {
-    const uint32_t band = place / (4u * w), r = place - band * 4u * w;
-    if (4u * band + 4u > h) return place;
-    const uint32_t tiles = w / 8u, t = r / 32u, k = r % 32u;
-    if (t < tiles) return (4u * band + k / 8u) * w + t * 8u + k % 8u;
-    const uint32_t rest = w - tiles * 8u, q = r - tiles * 32u;
-    return (4u * band + q / rest) * w + tiles * 8u + q % rest;
 }
 
 // camera::get_ray (camera.cpp:14-39)

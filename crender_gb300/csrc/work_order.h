@@ -1,0 +1,30 @@
+// work_order.h — in which order and shares the kernels take their work: plain
+// functions, also compiled by the host compiler for their tests.
+#pragma once
+
+#include <cstdint>
+
+#ifdef __CUDACC__
+#define CRG_HD __host__ __device__ __forceinline__
+#else
+#define CRG_HD inline
+#endif
+
+namespace crg {
+
+// Pixel at `place` of an image's order of work: 8 x 4 tiles, so that the 32 lanes
+// of a warp start on a compact patch, whose rays share nodes for longer than a
+// row's.  Tiles run along bands of four rows, then come the columns right of the
+// last full tile; a last band of fewer than four rows goes row by row, as does an
+// image of fewer (four rows of its width may not fit 32 bits).
+CRG_HD uint32_t tile_pixel(uint32_t place, uint32_t w, uint32_t h) {
+    if (h < 4u) return place;
+    const uint32_t band = place / (4u * w), r = place - band * 4u * w;
+    if (4u * band + 4u > h) return place;
+    const uint32_t tiles = w / 8u, t = r / 32u, k = r % 32u;
+    if (t < tiles) return (4u * band + k / 8u) * w + t * 8u + k % 8u;
+    const uint32_t rest = w - tiles * 8u, q = r - tiles * 32u;
+    return (4u * band + q / rest) * w + tiles * 8u + q % rest;
+}
+
+} // namespace crg

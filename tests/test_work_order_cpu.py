@@ -1,0 +1,50 @@
+"""The kernels' order of work (csrc/work_order.h), compiled by the host compiler."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "crender_gb300", "csrc")
+
+SOURCE = """
+#include "work_order.h"
+extern "C" void tile_pixels(const uint32_t *place, uint32_t n, uint32_t w, uint32_t h, uint32_t *out) {
+    for (uint32_t i = 0; i < n; ++i) out[i] = crg::tile_pixel(place[i], w, h);
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    d = tmp_path_factory.mktemp("work_order")
+    (d / "w.cpp").write_text(SOURCE)
+    subprocess.run([os.environ.get("CXX", "g++"), "-std=c++17", "-O1", "-shared", "-fPIC", "-I", CSRC, str(d / "w.cpp"), "-o",
+                    str(d / "w.so")], check=True)
+    return C.CDLL(str(d / "w.so"))
+
+
+def tile_pixels(lib, places, w, h):
+    places = np.ascontiguousarray(places, np.uint32)
+    out = np.empty_like(places)
+    lib.tile_pixels(places.ctypes.data_as(C.c_void_p), C.c_uint32(len(places)), C.c_uint32(w), C.c_uint32(h),
+                    out.ctypes.data_as(C.c_void_p))
+    return out
+
+
+@pytest.mark.parametrize("size", [(1, 1), (1, 9), (7, 3), (7, 4), (8, 4), (9, 5), (33, 6), (40, 12), (403, 301)])
+def test_tiles_cover_every_pixel_once(lib, size):
+    w, h = size
+    assert np.array_equal(np.sort(tile_pixels(lib, np.arange(w * h), w, h)), np.arange(w * h))
+
+
+@pytest.mark.parametrize("size", [(1 << 29, 4), ((1 << 29) - 3, 4), (1 << 30, 2), ((1 << 30) + 1, 1), (1 << 30, 1), (1 << 31, 1),
+                                  (3, 715827882)])
+def test_tiles_of_the_largest_films_stay_inside(lib, size):
+    """Up to 2^31 pixels, where four rows of the widest images no longer fit 32 bits."""
+    w, h = size
+    n = w * h
+    places = np.r_[0:64, n // 2:n // 2 + 64, n - 64:n]
+    out = tile_pixels(lib, places, w, h)
+    assert (out < n).all() and len(np.unique(out)) == len(places)
