@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(128, 4) k_adjoint(SceneDev S, CamDev cam, crg_
     // as the forward kernel: 8 x 4 pixel tiles, and with kSplitSpp samples or more a block's warps
     // replay a quarter of them each for the same 32 pixels
     const uint32_t parts = set.spp >= kSplitSpp ? 4u : 1u;
-    const uint32_t part = parts == 4u ? threadIdx.x >> 5 : 0u, quarter = (set.spp + parts - 1u) / parts;
+    const uint32_t part = parts == 4u ? threadIdx.x >> 5 : 0u;
     const uint32_t place = parts == 4u ? blockIdx.x * 32u + (threadIdx.x & 31u) : blockIdx.x * 128u + threadIdx.x;
     const uint32_t Wd = set.width, Hd = set.height;
     const bool inside = place < Wd * Hd;
@@ -178,8 +178,9 @@ __global__ void __launch_bounds__(128, 4) k_adjoint(SceneDev S, CamDev cam, crg_
     PathState ps;
     path_start(ps, mk(0, 0, 0), mk(0, 0, 1));
     // one loop over segments with path regeneration, as in the forward megakernel
-    const uint32_t end = min(set.spp, (part + 1u) * quarter);
-    uint32_t s = live ? min(set.spp, part * quarter) : end, i = 0;
+    uint32_t s, end, i = 0;
+    sample_share(set.spp, parts, part, s, end);
+    if (!live) s = end;
     while (__any_sync(0xFFFFFFFFu, s < end)) {
         const bool alive = s < end;
         if (alive && i == 0) {

@@ -27,4 +27,12 @@ CRG_HD uint32_t tile_pixel(uint32_t place, uint32_t w, uint32_t h) {
     return (4u * band + q / rest) * w + tiles * 8u + q % rest;
 }
 
+// Samples [begin, end) of `spp` that part `part` of `parts` takes, as even as whole
+// samples allow, the later parts less.
+CRG_HD void sample_share(uint32_t spp, uint32_t parts, uint32_t part, uint32_t &begin, uint32_t &end) {
+    const uint32_t share = spp / parts + (spp % parts ? 1u : 0u);
+    begin = part * share < spp ? part * share : spp;
+    end = begin + (spp - begin < share ? spp - begin : share);
+}
+
 } // namespace crg

@@ -13,6 +13,9 @@ SOURCE = """
 extern "C" void tile_pixels(const uint32_t *place, uint32_t n, uint32_t w, uint32_t h, uint32_t *out) {
     for (uint32_t i = 0; i < n; ++i) out[i] = crg::tile_pixel(place[i], w, h);
 }
+extern "C" void sample_share(uint32_t spp, uint32_t parts, uint32_t part, uint32_t *out) {
+    crg::sample_share(spp, parts, part, out[0], out[1]);
+}
 """
 
 
@@ -48,3 +51,15 @@ def test_tiles_of_the_largest_films_stay_inside(lib, size):
     places = np.r_[0:64, n // 2:n // 2 + 64, n - 64:n]
     out = tile_pixels(lib, places, w, h)
     assert (out < n).all() and len(np.unique(out)) == len(places)
+
+
+@pytest.mark.parametrize("parts", [1, 4])
+@pytest.mark.parametrize("spp", [1, 3, 4, 5, 8, 9, 131, (1 << 31) + 1, (1 << 32) - 5, (1 << 32) - 3, (1 << 32) - 1])
+def test_sample_shares_follow_one_another(lib, spp, parts):
+    at = 0
+    for part in range(parts):
+        out = (C.c_uint32 * 2)()
+        lib.sample_share(C.c_uint32(spp), C.c_uint32(parts), C.c_uint32(part), out)
+        assert out[0] == at and out[0] <= out[1] <= spp and out[1] - out[0] <= -(-spp // parts)
+        at = out[1]
+    assert at == spp
