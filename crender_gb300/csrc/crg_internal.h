@@ -153,9 +153,11 @@ void noalloc_prepare();
 constexpr uint32_t kTlasLeaf = 0x80000000u;
 
 // traverse.cu
+// `traversal`: a crg_traversal to keep to, or the one that suits the number of rays.
+constexpr int kTraversalBySize = -1;
 crg_status launch_intersect(const crg_scene *s, const crg_ray *rays, crg_hit *hits, uint32_t *occluded,
                             uint32_t *nodes, uint32_t *tris, uint64_t n, bool any, cudaStream_t stream,
-                            int traversal = CRG_TRAVERSAL_THREAD);
+                            int traversal = kTraversalBySize);
 
 // render.cu
 struct CamDev {

@@ -337,18 +337,10 @@ void launch_warp(const crg_scene *s, const crg_ray *rays, crg_hit *hits, uint32_
                                                         (uint32_t)n, 0u, (uint32_t *)s->err.ptr);
 }
 
-// Few rays leave the GPU idle whatever runs them, and a call lasts as long as its
-// longest ray's chain of steps.  W lanes to a ray make each step short (a child
-// box per lane), and a warp to a ray keeps the rays of a warp from waiting for
-// each other's branches: soup, 4,000 closest hits 107 -> 64 us, 127 on a mesh of
-// 11,520 triangles 30 -> 21, at width 2 1,000 on the soup 670 -> 461.  More rays
-// than warps that are resident together share them: 8,000 on the mesh take 39 us
-// at one to a warp, 34 at two and 39 a lane each, 16,000 take 37 at four and 40.
-constexpr uint64_t kFewRays = 4096;
-
+// One call of few rays (few_rays_per_warp): every warp has its own.
 template <int W>
-void launch_few(const crg_scene *s, const crg_ray *rays, crg_hit *hits, uint32_t *occluded, uint64_t n, bool any, cudaStream_t st) {
-    const uint32_t per_warp = n <= kFewRays ? 1u : n <= 2 * kFewRays ? 2u : 4u;
+void launch_few(const crg_scene *s, const crg_ray *rays, crg_hit *hits, uint32_t *occluded, uint64_t n, uint32_t per_warp, bool any,
+                cudaStream_t st) {
     const uint32_t grid = (uint32_t)((n + 4 * per_warp - 1) / (4 * per_warp));
     const uint4 *nd = (const uint4 *)s->wide.ptr;
     const float4 *tr = (const float4 *)s->tris.ptr;
@@ -363,7 +355,7 @@ void launch_few(const crg_scene *s, const crg_ray *rays, crg_hit *hits, uint32_t
 
 template <int W>
 void launch_w(const crg_scene *s, const crg_ray *rays, crg_hit *hits, uint32_t *occluded, uint32_t *nodes, uint32_t *tris,
-              uint64_t n, bool any, cudaStream_t st) {
+              uint64_t n, bool any, bool lanes, cudaStream_t st) {
     if (s->ninst && s->ntri > 0) {
         const rc::SceneDev S = rc::scene_dev(s);
         const uint64_t blocks = (n + 127) / 128;
@@ -373,8 +365,8 @@ void launch_w(const crg_scene *s, const crg_ray *rays, crg_hit *hits, uint32_t *
         if (tris) cudaMemsetAsync(tris, 0, 4 * n, st);
         return;
     }
-    if (n <= (W == 8 ? 4 * kFewRays : kFewRays) && s->ntri > 0 && !nodes && !tris) {
-        launch_few<W>(s, rays, hits, occluded, n, any, st);
+    if (const uint32_t per_warp = few_rays_per_warp(n, W, s->ntri, lanes || nodes || tris)) {
+        launch_few<W>(s, rays, hits, occluded, n, per_warp, any, st);
         return;
     }
     // a block's run of rays: long enough that its warps mostly run full, short
@@ -413,10 +405,11 @@ crg_status launch_intersect(const crg_scene *s, const crg_ray *rays, crg_hit *hi
         if (e != cudaSuccess) return cuda_error(s->ctx, e, "k_intersect_warp launch");
         return CRG_OK;
     }
+    const bool lanes = traversal == CRG_TRAVERSAL_THREAD;
     switch (s->width) {
-    case 2: launch_w<2>(s, rays, hits, occluded, nodes, tris, n, any, st); break;
-    case 4: launch_w<4>(s, rays, hits, occluded, nodes, tris, n, any, st); break;
-    default: launch_w<8>(s, rays, hits, occluded, nodes, tris, n, any, st); break;
+    case 2: launch_w<2>(s, rays, hits, occluded, nodes, tris, n, any, lanes, st); break;
+    case 4: launch_w<4>(s, rays, hits, occluded, nodes, tris, n, any, lanes, st); break;
+    default: launch_w<8>(s, rays, hits, occluded, nodes, tris, n, any, lanes, st); break;
     }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_error(s->ctx, e, "k_intersect launch");

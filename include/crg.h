@@ -400,15 +400,15 @@ crg_status crg_intersect_closest_counted(const crg_scene *scene, const crg_ray *
                                          crg_stream stream);
 
 /* Traversal schemes of the batched queries (the results are the same):
- *   THREAD: one ray per thread, its group stack in local memory (the default
- *           of crg_intersect_closest / crg_intersect_any; calls of a few
- *           thousand rays take WARP's steps, without its refill);
+ *   THREAD: one ray per thread, its group stack in local memory;
  *   WARP:   W lanes per ray (W = the BVH width), 32 / W rays per warp: the
  *           ray's node is read with 16-byte vector loads by its lanes into
  *           shared memory, each lane tests one child box, pending triangles
  *           are tested W at a time, and each ray's group stack lives in its
  *           warp's shared memory.  Scenes traced through placements use
- *           THREAD. */
+ *           THREAD.
+ * crg_intersect_closest / crg_intersect_any take THREAD, except that calls of a
+ * few thousand rays take WARP's steps without its refill. */
 typedef enum crg_traversal { CRG_TRAVERSAL_THREAD = 0, CRG_TRAVERSAL_WARP = 1 } crg_traversal;
 /* crg_intersect_closest / crg_intersect_any with an explicit traversal scheme. */
 crg_status crg_intersect_closest_with(const crg_scene *scene, const crg_ray *d_rays, crg_hit *d_hits, uint64_t n,

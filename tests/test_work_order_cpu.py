@@ -16,6 +16,9 @@ extern "C" void tile_pixels(const uint32_t *place, uint32_t n, uint32_t w, uint3
 extern "C" void sample_share(uint32_t spp, uint32_t parts, uint32_t part, uint32_t *out) {
     crg::sample_share(spp, parts, part, out[0], out[1]);
 }
+extern "C" uint32_t few_rays_per_warp(uint64_t n, uint32_t width, uint32_t ntri, uint32_t lanes) {
+    return crg::few_rays_per_warp(n, width, ntri, lanes != 0);
+}
 """
 
 
@@ -63,3 +66,13 @@ def test_sample_shares_follow_one_another(lib, spp, parts):
         assert out[0] == at and out[0] <= out[1] <= spp and out[1] - out[0] <= -(-spp // parts)
         at = out[1]
     assert at == spp
+
+
+@pytest.mark.parametrize("width", [2, 4, 8])
+def test_few_rays_share_a_warp_unless_lanes_are_asked_for(lib, width):
+    few = lambda n, ntri=10, lanes=0: lib.few_rays_per_warp(C.c_uint64(n), width, ntri, lanes)
+    assert [few(n) for n in (1, 4096)] == [1, 1]
+    assert [few(n) for n in (4097, 8192, 8193, 16384)] == ([2, 2, 4, 4] if width == 8 else [0] * 4)
+    assert few(16385) == few(1 << 33) == 0
+    assert few(1, ntri=0) == 0
+    assert not any(few(n, lanes=1) for n in (1, 4096, 8192, 16384))
