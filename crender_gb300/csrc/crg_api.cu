@@ -1388,7 +1388,7 @@ crg_status batch_call(crg_scene *const *scenes, uint32_t nscenes, const crg_view
     // defaults: up to 128M paths in flight (about 20 GB of path state for a batch that large; a
     // frame never holds more paths than its largest chunk's samples), 128M-sample chunks (2 GB of
     // sample slots), split stages with per-lane refill in the traversal stages
-    // (fuse 0: render_batch takes 1, or 3 for a small pool)
+    // (fuse 0: by default_fusion)
     crg_wavefront_opts o{1u << 27, 1u << 27, 128, 32, 0, 0, 0, 0, 16};
     if (opts) {
         if (opts->path_pool) o.path_pool = opts->path_pool;

@@ -793,10 +793,6 @@ struct Workspace {
     DevBuf buf;
 };
 
-// Paths in flight up to which a batch without a fusion level of its own runs one
-// kernel a bounce.
-constexpr uint32_t kFusedPaths = 1u << 19;
-
 size_t align_up(size_t x) { return (x + 255) / 256 * 256; }
 
 // Persistent grids: each per-bounce kernel fills every SM with as many of its
@@ -1392,11 +1388,8 @@ crg_status render_batch(crg_context *ctx, crg_scene *const *scenes, uint32_t nsc
         CRG_CUDA(ctx, cudaEventRecord(B->stage_ev[k], st));
     }
     // persistent grid: resident blocks of the launched kernels on every SM
-    // fusion level 0..2 (split with placements).  By default a small pool takes one kernel a bounce: its
-    // stages last as long as their longest ray's chain of steps, which fused they start only once.  Split /
-    // fused: 4,096 paths 320 / 245 us, 20K 767 / 616, 140K 1,032 / 822, 930K 1,634 / 1,571, 4M 3,280 / 3,865.
-    const uint32_t auto_fuse = P <= kFusedPaths && o.host_loop == 0 ? 2u : 0u;
-    const uint32_t fuse = instanced ? 0u : o.fuse ? o.fuse - 1 : auto_fuse;
+    // fusion level 0..2 (split with placements)
+    const uint32_t fuse = instanced ? 0u : (o.fuse ? o.fuse : default_fusion(P, max_chunk, o.host_loop)) - 1u;
     int per_sm = 0;
     {
         const uint64_t key = (uint64_t)width | (uint64_t)fuse << 8 | (uint64_t)o.block_size << 16 | 4ull << 40;

@@ -559,8 +559,9 @@ typedef struct crg_wavefront_opts {
                                same, timing every stage with CUDA events on the stream
                                (crg_batch_stage_times_get) */
     uint32_t fuse;          /* stage fusion (films are identical for every value; default 1, or 3
-                               when at most 2^19 paths are in flight and block_size,
-                               fetch, refill and host_loop are 0):
+                               when at most 2^19 paths are in flight, 2^17 if the pool is
+                               smaller than a chunk, with block_size, fetch, refill and
+                               host_loop 0):
                                1 = separate extend / shade / shadow kernels and queues;
                                2 = the shadow test runs inside shade (no shadow queue);
                                3 = extend + shade + shadow in one kernel per bounce */

@@ -16,6 +16,9 @@ extern "C" void tile_pixels(const uint32_t *place, uint32_t n, uint32_t w, uint3
 extern "C" void sample_share(uint32_t spp, uint32_t parts, uint32_t part, uint32_t *out) {
     crg::sample_share(spp, parts, part, out[0], out[1]);
 }
+extern "C" uint32_t default_fusion(uint64_t pool, uint64_t largest_chunk, uint32_t host_loop) {
+    return crg::default_fusion(pool, largest_chunk, host_loop);
+}
 extern "C" uint32_t few_rays_per_warp(uint64_t n, uint32_t width, uint32_t ntri, uint32_t lanes) {
     return crg::few_rays_per_warp(n, width, ntri, lanes != 0);
 }
@@ -76,3 +79,10 @@ def test_few_rays_share_a_warp_unless_lanes_are_asked_for(lib, width):
     assert few(16385) == few(1 << 33) == 0
     assert few(1, ntri=0) == 0
     assert not any(few(n, lanes=1) for n in (1, 4096, 8192, 16384))
+
+
+def test_default_fusion_goes_by_the_pool_and_its_refills(lib):
+    fuse = lambda pool, chunk, loop=0: lib.default_fusion(C.c_uint64(pool), C.c_uint64(chunk), loop)
+    assert [fuse(p, p) for p in (1, 1 << 19, (1 << 19) + 1, 1 << 27)] == [3, 3, 1, 1]
+    assert [fuse(p, 1 << 24) for p in (1, 1 << 17, (1 << 17) + 1, 1 << 19)] == [3, 3, 1, 1]
+    assert [fuse(1000, 1000, loop) for loop in (0, 1, 2)] == [3, 1, 1]
