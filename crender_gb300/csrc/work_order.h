@@ -60,9 +60,9 @@ CRG_HD uint32_t few_rays_per_warp(uint64_t n, uint32_t width, uint32_t ntri, boo
 // 1,634 / 1,571, 4M 3,280 / 3,865.  A pool refilled many times keeps its kernels
 // full, so the split stages win earlier: 16.8M samples of the 72K-triangle mesh at
 // 2^17 paths 51.5 / 51.3 ms, at 2^19 24.3 / 35.0 (the box 33.6 / 26.5 and 23.0 / 18.9).
-// Host-driven loops run the split stages.
+// Stage times are those of the split stages (host_loop 2).
 CRG_HD uint32_t default_fusion(uint64_t pool, uint64_t largest_chunk, uint32_t host_loop) {
-    return host_loop == 0u && pool <= (pool < largest_chunk ? 1u << 17 : 1u << 19) ? 3u : 1u;
+    return host_loop != 2u && pool <= (pool < largest_chunk ? 1u << 17 : 1u << 19) ? 3u : 1u;
 }
 
 } // namespace crg

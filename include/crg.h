@@ -557,11 +557,12 @@ typedef struct crg_wavefront_opts {
     uint32_t host_loop;     /* 1 = drive the loop from the host instead of one graph with a
                                device-side condition (same kernels; for profilers); 2 = the
                                same, timing every stage with CUDA events on the stream
-                               (crg_batch_stage_times_get) */
+                               (crg_batch_stage_times_get; with fuse 0 always the split
+                               stages, also where 0 and 1 fuse them) */
     uint32_t fuse;          /* stage fusion (films are identical for every value; default 1, or 3
                                when at most 2^19 paths are in flight, 2^17 if the pool is
-                               smaller than a chunk, with block_size, fetch, refill and
-                               host_loop 0):
+                               smaller than a chunk, with block_size, fetch and refill 0
+                               and host_loop not 2):
                                1 = separate extend / shade / shadow kernels and queues;
                                2 = the shadow test runs inside shade (no shadow queue);
                                3 = extend + shade + shadow in one kernel per bounce */

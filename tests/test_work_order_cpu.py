@@ -85,4 +85,4 @@ def test_default_fusion_goes_by_the_pool_and_its_refills(lib):
     fuse = lambda pool, chunk, loop=0: lib.default_fusion(C.c_uint64(pool), C.c_uint64(chunk), loop)
     assert [fuse(p, p) for p in (1, 1 << 19, (1 << 19) + 1, 1 << 27)] == [3, 3, 1, 1]
     assert [fuse(p, 1 << 24) for p in (1, 1 << 17, (1 << 17) + 1, 1 << 19)] == [3, 3, 1, 1]
-    assert [fuse(1000, 1000, loop) for loop in (0, 1, 2)] == [3, 1, 1]
+    assert [fuse(1000, 1000, loop) for loop in (0, 1, 2)] == [3, 3, 1]
