@@ -45,9 +45,11 @@ CRG_HD void sample_share(uint32_t spp, uint32_t parts, uint32_t part, uint32_t &
 // 11,520 triangles 30 -> 21, at width 2 1,000 on the soup 670 -> 461.  More rays
 // than warps that are resident together share them: 8,000 on the mesh take 39 us
 // at one to a warp, 34 at two and 39 a lane each, 16,000 take 37 at four and 40.
+// Two lanes to a ray gain little on a step: below 32 rays they lose more than the
+// company costs (10K triangles at width 2: one ray 49 against 35 us, 32 rays 74 against 86).
 constexpr uint64_t kFewRays = 4096;
 CRG_HD uint32_t few_rays_per_warp(uint64_t n, uint32_t width, uint32_t ntri, bool lanes) {
-    if (lanes || ntri == 0u || n > (width == 8u ? 4u * kFewRays : kFewRays)) return 0u;
+    if (lanes || ntri == 0u || (width == 2u && n < 32u) || n > (width == 8u ? 4u * kFewRays : kFewRays)) return 0u;
     return n <= kFewRays ? 1u : n <= 2u * kFewRays ? 2u : 4u;
 }
 

@@ -74,7 +74,7 @@ def test_sample_shares_follow_one_another(lib, spp, parts):
 @pytest.mark.parametrize("width", [2, 4, 8])
 def test_few_rays_share_a_warp_unless_lanes_are_asked_for(lib, width):
     few = lambda n, ntri=10, lanes=0: lib.few_rays_per_warp(C.c_uint64(n), width, ntri, lanes)
-    assert [few(n) for n in (1, 4096)] == [1, 1]
+    assert [few(n) for n in (1, 31, 32, 4096)] == ([0, 0, 1, 1] if width == 2 else [1, 1, 1, 1])
     assert [few(n) for n in (4097, 8192, 8193, 16384)] == ([2, 2, 4, 4] if width == 8 else [0] * 4)
     assert few(16385) == few(1 << 33) == 0
     assert few(1, ntri=0) == 0
