@@ -588,7 +588,8 @@ __device__ void optimize_treelet(const Tree &T, uint32_t r, uint32_t left, uint3
     }
     __syncwarp();
     {
-        // a lane's four subsets share its choice of the first five leaves
+        // a lane's four subsets share its choice of the first five leaves; leaves are merged in their
+        // order (it counts where a corner is a NaN)
         Box b{{INFINITY, INFINITY, INFINITY}, {-INFINITY, -INFINITY, -INFINITY}};
         auto with = [&](const Box &x, int j) {
             const float4 lo = w.lo[j], hi = w.hi[j];
@@ -599,11 +600,11 @@ __device__ void optimize_treelet(const Tree &T, uint32_t r, uint32_t left, uint3
             if (j < nl && (lane >> j) & 1u) b = with(b, j);
         w.aS[lane] = area(b);
         if (nl >= 6) {
-            w.aS[lane + 32] = area(with(b, 5));
+            const Box b5 = with(b, 5);
+            w.aS[lane + 32] = area(b5);
             if (nl >= 7) {
-                const Box b6 = with(b, 6);
-                w.aS[lane + 64] = area(b6);
-                w.aS[lane + 96] = area(with(b6, 5));
+                w.aS[lane + 64] = area(with(b, 6));
+                w.aS[lane + 96] = area(with(b5, 6));
             }
         }
     }
@@ -826,7 +827,26 @@ __device__ __forceinline__ uint32_t group_top(uint32_t key, uint32_t &who) {
     return top;
 }
 
-__device__ __forceinline__ Box group_merge(Box b) {
+// Box of a group's children, lane i holding child i.  The corners' minima and maxima
+// may be taken in any order unless one is a NaN, which the next child replaces: then
+// the children are merged one after the other, as the CPU form does.
+__device__ __forceinline__ Box group_merge(Box b, bool child) {
+    bool nan = false;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) nan = nan || b.lo[a] != b.lo[a] || b.hi[a] != b.hi[a];
+    if (__any_sync(0xFFFFFFFFu, child && nan)) {
+        Box r = b;
+        for (int j = 0; j < 8; ++j) {
+            Box o;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                o.lo[a] = __shfl_sync(0xFFFFFFFFu, b.lo[a], j, 8);
+                o.hi[a] = __shfl_sync(0xFFFFFFFFu, b.hi[a], j, 8);
+            }
+            if (__shfl_sync(0xFFFFFFFFu, child, j, 8)) r = j ? merge(r, o) : o;
+        }
+        return r;
+    }
 #pragma unroll
     for (int off = 4; off >= 1; off >>= 1)
 #pragma unroll
@@ -894,28 +914,44 @@ __global__ void __launch_bounds__(kLevelThreads) k_level_open(Collapse C, const 
         const bool child = c < m;
         // octant codes: repeatedly the largest projection of a child's centre (seen from the
         // node's) on a free octant's diagonal; the first child, then the first code, of equals
-        const Box nb = group_merge(e.b);
-        float off[3], score[8];
+        const Box nb = group_merge(e.b, child);
+        float off[3];
+        uint32_t score[8]; // by order-preserving key; 0: not a number
 #pragma unroll
         for (int a = 0; a < 3; ++a) off[a] = (e.b.lo[a] + e.b.hi[a]) * 0.5f - (nb.lo[a] + nb.hi[a]) * 0.5f;
+        bool nan = false;
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             const float sx = (q & 4) ? -1.0f : 1.0f, sy = (q & 2) ? -1.0f : 1.0f, sz = (q & 1) ? -1.0f : 1.0f;
-            score[q] = (off[0] * sx + off[1] * sy) + off[2] * sz;
+            const float s = (off[0] * sx + off[1] * sy) + off[2] * sz;
+            score[q] = s == s ? f2key(s + 0.0f) : 0u; // + 0: no negative zero
+            nan = nan || s != s;
         }
+        const bool odd = __any_sync(0xFFFFFFFFu, child && nan);
         uint32_t used = 0u, code = 0u;
         bool placed = !child;
         for (uint32_t it = 0; it < C.W; ++it) {
-            float bs = 0.0f;
-            uint32_t bc = 8u;
+            uint32_t bs = 0u, bc = 0u;
 #pragma unroll
             for (uint32_t q = 0; q < 8; ++q)
-                if (!(used & (1u << q)) && (bc == 8u || score[q] > bs)) {
+                if (!(used & (1u << q)) && score[q] > bs) {
                     bs = score[q];
                     bc = q;
                 }
+            if (odd) {
+                // the first child's first code stands against any other if it is not a number
+                const uint32_t open = __ballot_sync(0xFFFFFFFFu, !placed) >> (threadIdx.x & 24u) & 0xFFu;
+                const uint32_t q0 = (uint32_t)__ffs(~used) - 1u;
+                bool none = false;
+#pragma unroll
+                for (uint32_t q = 0; q < 8; ++q) none = none || (q == q0 && score[q] == 0u);
+                if (none && (open & (0u - open)) == 1u << c) {
+                    bs = 0xFFFFFFFFu;
+                    bc = q0;
+                }
+            }
             uint32_t who;
-            const uint32_t top = group_top(placed ? 0u : max(f2key(bs + 0.0f), 1u), who); // + 0: no negative zero
+            const uint32_t top = group_top(placed ? 0u : bs, who);
             const uint32_t q = __shfl_sync(0xFFFFFFFFu, bc, (int)who, 8);
             if (top != 0u) {
                 used |= 1u << q;
@@ -1071,7 +1107,7 @@ __global__ void __launch_bounds__(kLevelThreads) k_emit(Collapse C, const LevelS
         const uint32_t code = q & 7u, cnt = leafslot ? q >> 4 : 0u;
         Box b{{INFINITY, INFINITY, INFINITY}, {-INFINITY, -INFINITY, -INFINITY}};
         if (child) b = level_child(C.T, ref).b;
-        const Box nb = group_merge(b);
+        const Box nb = group_merge(b, child);
         // the frame of axis a, on lane a
         int ex = 0;
         float pf = 0.0f;
