@@ -1337,7 +1337,8 @@ crg_status build_pipeline(const BvhTarget &t, const crg_build_opts &o, ScratchSo
             // where it does not: its treelets wait for one another, those of different warps do not.
             // Three rounds over 10,007 triangles and the rest of the build 574 us with 32 leaves, 540 with
             // 8, 511 with 2, 517 with 1; 33,282 triangles, two builds, 1.355 ms with 32, 1.300 with 4;
-            // 163,282 triangles 1.71 ms with 32, 1.72 with 16, 1.76 with 8.
+            // 163,282 triangles 1.71 ms with 32, 1.72 with 16, 1.76 with 8.  (152 SMs x 32 warps: the GPU that
+            // this was measured on; any value gives the same tree.)
             uint32_t gamma = 7, per = 32;
             while (per > 2u && n / per < 152u * 32u) per /= 2u;
             for (uint32_t round = 0; round < o.treelet_rounds; ++round) {

@@ -519,7 +519,7 @@ __device__ __forceinline__ void lane_init(LaneTrav &T, const RayPre &r, float tm
 // Tests the pending triangles of the warp's lanes (all 32 lanes call it; a
 // lane without a ray has none), in windows of 32 pairs.
 template <bool ANY>
-__device__ __forceinline__ void warp_tris(LaneTrav &T, WarpRays &sh, const float4 *__restrict__ tris) {
+__device__ __forceinline__ void warp_tris(LaneTrav &T, WarpRays &sh) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t cnt = (uint32_t)__popc(T.tg.y);
     if (__ballot_sync(0xFFFFFFFFu, cnt != 0u) == 0u) return;
@@ -629,7 +629,7 @@ __device__ __forceinline__ void warp_traverse(bool on, bool any, const RayPre &r
         if ((uint32_t)__popc(visitors) < kVisitors) {
             // few lanes to visit with: the triangle tests first, if there are any
             if (__any_sync(0xFFFFFFFFu, T.tg.y != 0u)) {
-                warp_tris<false>(T, sh, tris);
+                warp_tris<false>(T, sh);
                 if (any && on && T.best_prim != 0xFFFFFFFFu) T.ng.y = 0u;
                 continue;
             }
@@ -726,7 +726,7 @@ __device__ __forceinline__ void dyn_traverse(WarpRays &sh, Take &&take, unsigned
                 }
             }
         }
-        warp_tris<ANY>(T, sh, tris);
+        warp_tris<ANY>(T, sh);
         if (ANY && T.occluded) T.ng.y = 0u;
         if (state == kRun && T.ng.y < 1u << 24) state = kEnded;
     }

@@ -53,7 +53,7 @@ using namespace rc;
 
 namespace {
 
-// MINB: blocks of 128 threads per SM, see launch_w.
+// MINB: blocks of 128 threads per SM, see render_form.
 // PL: how the scene's placements are traced (warp_trace).
 //
 // A warp traces its lanes' segments together and then their shadow tests, sharing
@@ -253,17 +253,9 @@ void launch_m(const SceneDev &S, const CamDev &cam, const crg_settings &set, con
 template <int W>
 void launch_w(const SceneDev &S, const CamDev &cam, const crg_settings &set, const FilmDev &F, uint64_t spp0, int sm_count,
               cudaStream_t st) {
-    // A few triangles lie in L1 and the kernel is bound by issue: six blocks per SM (80 registers; 12.7 ms
-    // on the box's 36 triangles, 13.9 at eight); more wait on loads: eight (64 registers; 4.63 against 4.67
-    // ms at 1,602 triangles, 7.06 against 7.41 at 33K, 12.65 against 13.59 at 4.2M).
-    const bool small = S.ntri < 1024u;
-    // Splitting a pixel's samples fills the GPU with a quarter of the pixels, evens out the end of the
-    // launch and keeps a tile's rays in one SM's L1: mesh 1920x1080x4 12.4 -> 11.6 ms, 174x136x229 98 ->
-    // 35, box 65x70x256 14.7 -> 4.6, 517x333x64 6.3 -> 5.9.  A view of a small scene that fills the GPU
-    // four times only pays for the rounds (box 800x600x16 4.45 -> 4.59, 1920x1080x16 13.1 -> 14.7); from
-    // twice on it goes either way by the view (512x512x64 11.8 -> 12.4, 700x500x64 13.3 -> 12.6).
-    const uint64_t wave = 6ull * (uint64_t)(sm_count > 0 ? sm_count : 1) * 128ull;
-    const bool split = set.spp >= 4 && !(small && !S.ninst && (uint64_t)set.width * set.height >= 4 * wave);
+    const uint64_t npix = (uint64_t)set.width * set.height;
+    const RenderForm form = render_form(npix, set.spp, S.ntri, S.ninst != 0, (uint32_t)(sm_count > 0 ? sm_count : 1));
+    const bool split = form.split;
     if (S.counters) { // the instrumented variants: one form per kind of scene
         if (S.ninst > kLoopPlacements) launch_m<W, 4, 2, false, true>(S, cam, set, F, spp0, st);
         else if (S.ninst) launch_m<W, 4, 1, false, true>(S, cam, set, F, spp0, st);
@@ -274,7 +266,7 @@ void launch_w(const SceneDev &S, const CamDev &cam, const crg_settings &set, con
     } else if (S.ninst) {
         if (split) launch_m<W, 4, 1, true>(S, cam, set, F, spp0, st);
         else launch_m<W, 4, 1, false>(S, cam, set, F, spp0, st);
-    } else if (small) {
+    } else if (form.blocks == 6u) {
         if (split) launch_m<W, 6, 0, true>(S, cam, set, F, spp0, st);
         else launch_m<W, 6, 0, false>(S, cam, set, F, spp0, st);
     } else {

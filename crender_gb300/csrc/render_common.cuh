@@ -539,7 +539,8 @@ __device__ __forceinline__ bool occluded(const SceneDev &S, v3 o, v3 d, float tm
 // says whether the lane has a ray.  The answers are those of closest_t and
 // occluded_t: PL 0 traces a scene of one mesh, 1 its placements by the plain
 // loop, 2 through the top-level tree, one placement per lane at a time.  Any hit:
-// h.prim is a primitive or 0xFFFFFFFF.
+// h.prim is a primitive or 0xFFFFFFFF.  h.u and h.v stay as they are: shading forms
+// the barycentrics again where it needs them.
 template <int W, bool CNT, int PL>
 __device__ __forceinline__ void warp_trace(const SceneDev &S, WarpRays &sh, bool on, bool any, v3 o, v3 d, float tmax, Hit &h,
                                            PathCtx &C) {
@@ -612,7 +613,6 @@ __device__ __forceinline__ void warp_trace(const SceneDev &S, WarpRays &sh, bool
         }
         if (PL == 2 && had && !wk.ok) C.err = 1u;
     }
-    h.u = h.v = 0.0f;
     if (CNT) {
         C.nodes += st.nodes;
         C.tris += st.tris;

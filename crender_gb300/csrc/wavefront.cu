@@ -797,8 +797,9 @@ size_t align_up(size_t x) { return (x + 255) / 256 * 256; }
 
 // Persistent grids: each per-bounce kernel fills every SM with as many of its
 // own blocks as fit (the traversal kernels need fewer registers than shading,
-// so they get more warps to hide memory latency); work is fetched atomically,
-// so any grid size is correct.
+// so they get more warps to hide memory latency).  Work is fetched atomically or,
+// in split shading, by the warp's place in the grid: any grid size is correct as
+// long as a stage that has nothing to do finds its queue empty (wf_control).
 struct Grids {
     uint32_t ext, shade, shadow;
 };

@@ -53,6 +53,42 @@ CRG_HD uint32_t few_rays_per_warp(uint64_t n, uint32_t width, uint32_t ntri, boo
     return n <= kFewRays ? 1u : n <= 2u * kFewRays ? 2u : 4u;
 }
 
+// Form of the megakernel for an image: a pixel's samples split over a block's four
+// warps or not, and blocks of 128 threads per SM (4 with placements).
+//
+// Blocks: a few triangles lie in L1 and the kernel is bound by issue: six (80
+// registers; 12.7 ms on the box's 36 triangles, 13.9 at eight); more wait on loads:
+// eight (64 registers; 4.63 against 4.67 ms at 1,602 triangles, 7.06 against 7.41 at
+// 33K, 12.65 against 13.59 at 4.2M), but six where those hold the whole image at
+// once, which gains nothing from more and loses what spills cost (72K triangles
+// 64x64x1 226 against 220 us, 100x75x1 269 / 261, 256x256x1 317 / 307).
+//
+// Split: a quarter of the pixels then fills the GPU, the end of the launch is evened
+// out and a tile's rays stay in one SM's L1: mesh 1920x1080x4 12.4 -> 11.6 ms,
+// 174x136x229 98 -> 35, box 65x70x256 14.7 -> 4.6, 517x333x64 6.3 -> 5.9.  A view of a
+// small scene that fills the GPU four times only pays for the rounds (box 800x600x16
+// 4.45 -> 4.59, 1920x1080x16 13.1 -> 14.7); from twice on it goes either way by the
+// view (512x512x64 11.8 -> 12.4, 700x500x64 13.3 -> 12.6).  Two or three samples leave
+// warps of a block idle, so they are split only where all blocks run at once, or up to
+// four times as many where rays wait on memory: 72K triangles 64x64x2 366 -> 216 us
+// (327 on a traversal per thread), 64x64x3 532 -> 218 (505), 400x300x2 489 -> 334,
+// 640x480x2 637 -> 626, 1283x721x2 1,164 -> 1,340; six placements 160x120x2 254 -> 143,
+// 256x256x2 353 -> 406; the box 160x120x2 138 -> 86, 256x256x2 162 -> 186.
+struct RenderForm {
+    bool split;
+    uint32_t blocks;
+};
+CRG_HD RenderForm render_form(uint64_t npix, uint32_t spp, uint32_t ntri, bool placed, uint32_t sms) {
+    const bool small = ntri < 1024u;
+    const uint64_t wave = 6ull * sms * 128ull; // pixels that six blocks per SM hold, a lane each
+    RenderForm f{};
+    f.blocks = placed ? 4u : small ? 6u : 8u;
+    if (spp >= 4u) f.split = !(small && !placed && npix >= 4u * wave);
+    else f.split = spp >= 2u && npix <= (f.blocks == 8u ? 4u : 1u) * 32ull * f.blocks * sms;
+    if (f.blocks == 8u && npix * (f.split ? 4u : 1u) <= wave) f.blocks = 6u;
+    return f;
+}
+
 // Stage fusion (crg_wavefront_opts::fuse, 1 to 3) of a batch that asks for none, with
 // `pool` paths in flight and chunks of at most `largest_chunk` samples.
 //

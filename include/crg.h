@@ -549,7 +549,8 @@ typedef struct crg_wavefront_opts {
                                about 156 bytes of path state each) */
     uint32_t chunk_samples; /* samples resolved into the films per chunk (default 134,217,728) */
     uint32_t block_size;    /* threads per block of the persistent kernels: 64, 128 or 256 (default 128) */
-    uint32_t fetch;         /* queue entries a warp takes per atomic, multiple of 32 (default 32) */
+    uint32_t fetch;         /* queue entries a warp takes per atomic, multiple of 32 (default 32);
+                               the split shade stage takes its own by its place in the grid */
     uint32_t max_iterations;/* cap on the device-side loop (0 = a bound derived from the batch);
                                reaching it ends the frame with CRG_ERR_TIMEOUT */
     uint32_t count_work;    /* 1 = instrumented kernels: crg_batch_stats_get also reports
