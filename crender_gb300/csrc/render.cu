@@ -78,8 +78,9 @@ template <int PL, bool SPLIT> constexpr uint32_t kRenderThreads = SPLIT || PL ? 
 
 template <int W, int MODE, bool CNT, int MINB, int PL, bool SPLIT>
 __global__ void __launch_bounds__((kRenderThreads<PL, SPLIT>), MINB * 128 / kRenderThreads<PL, SPLIT>)
-k_render(SceneDev S, CamDev cam, crg_settings set, FilmDev F, uint64_t spp0) {
+k_render(SceneDev S, CamDev cam, crg_settings set, FilmDev F, uint64_t spp0, uint32_t pixels) {
     constexpr uint32_t T = kRenderThreads<PL, SPLIT>;
+    constexpr bool kOwnBlock = T == 32u; // a warp with its pixels to itself, `pixels` of them
     __shared__ WarpRays s_rays[T / 32];
     // SPLIT: the round's radiances [sample][channel][pixel]; else, for films with FP64
     // planes, 6 sums per thread
@@ -87,9 +88,9 @@ k_render(SceneDev S, CamDev cam, crg_settings set, FilmDev F, uint64_t spp0) {
     float *s_round = reinterpret_cast<float *>(s_sums);
     WarpRays &sh = s_rays[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u, part = threadIdx.x >> 5;
-    const uint32_t place = SPLIT ? blockIdx.x * 32u + lane : blockIdx.x * T + threadIdx.x;
+    const uint32_t place = SPLIT ? blockIdx.x * 32u + lane : kOwnBlock ? blockIdx.x * pixels + lane : blockIdx.x * T + threadIdx.x;
     const uint32_t Wd = set.width, Hd = set.height;
-    const bool inside = place < Wd * Hd;
+    const bool inside = place < Wd * Hd && (!kOwnBlock || lane < pixels);
     const uint32_t pix = inside ? tile_pixel(place, Wd, Hd) : 0u;
     PathCtx C{pix, 0, set.seed, 0, 0, 0, 0ull, 0ull};
     const uint32_t px = pix % Wd, py = pix / Wd;
@@ -239,15 +240,16 @@ k_render(SceneDev S, CamDev cam, crg_settings set, FilmDev F, uint64_t spp0) {
 }
 
 template <int W, int MINB, int PL, bool SPLIT, bool CNT = false>
-void launch_m(const SceneDev &S, const CamDev &cam, const crg_settings &set, const FilmDev &F, uint64_t spp0, cudaStream_t st) {
+void launch_m(const SceneDev &S, const CamDev &cam, const crg_settings &set, const FilmDev &F, uint64_t spp0, cudaStream_t st,
+              uint32_t pixels = 32) {
     constexpr uint32_t T = kRenderThreads<PL, SPLIT>;
-    const uint32_t per_block = SPLIT ? 32 : T;
+    const uint32_t per_block = SPLIT ? 32 : T == 32 ? pixels : T;
     const uint32_t blocks = (uint32_t)(((uint64_t)set.width * set.height + per_block - 1) / per_block);
     const size_t shared = SPLIT ? sizeof(float) * 96 * (set.spp < kRound ? set.spp : kRound) : F.sum64 ? sizeof(double) * 6 * T : 0;
     if (set.mode == CRG_MODE_EXTENDED)
-        k_render<W, CRG_MODE_EXTENDED, CNT, MINB, PL, SPLIT><<<blocks, T, shared, st>>>(S, cam, set, F, spp0);
+        k_render<W, CRG_MODE_EXTENDED, CNT, MINB, PL, SPLIT><<<blocks, T, shared, st>>>(S, cam, set, F, spp0, pixels);
     else
-        k_render<W, CRG_MODE_FAITHFUL, CNT, MINB, PL, SPLIT><<<blocks, T, shared, st>>>(S, cam, set, F, spp0);
+        k_render<W, CRG_MODE_FAITHFUL, CNT, MINB, PL, SPLIT><<<blocks, T, shared, st>>>(S, cam, set, F, spp0, pixels);
 }
 
 template <int W>
@@ -268,10 +270,10 @@ void launch_w(const SceneDev &S, const CamDev &cam, const crg_settings &set, con
         else launch_m<W, 4, 1, false>(S, cam, set, F, spp0, st);
     } else if (form.blocks == 6u) {
         if (split) launch_m<W, 6, 0, true>(S, cam, set, F, spp0, st);
-        else launch_m<W, 6, 0, false>(S, cam, set, F, spp0, st);
+        else launch_m<W, 6, 0, false>(S, cam, set, F, spp0, st, form.pixels);
     } else {
         if (split) launch_m<W, 8, 0, true>(S, cam, set, F, spp0, st);
-        else launch_m<W, 8, 0, false>(S, cam, set, F, spp0, st);
+        else launch_m<W, 8, 0, false>(S, cam, set, F, spp0, st, form.pixels);
     }
 }
 

@@ -54,14 +54,16 @@ CRG_HD uint32_t few_rays_per_warp(uint64_t n, uint32_t width, uint32_t ntri, boo
 }
 
 // Form of the megakernel for an image: a pixel's samples split over a block's four
-// warps or not, and blocks of 128 threads per SM (4 with placements).
+// warps or not, blocks of 128 threads per SM (4 with placements), and pixels of a
+// warp where it has them to itself.
 //
 // Blocks: a few triangles lie in L1 and the kernel is bound by issue: six (80
 // registers; 12.7 ms on the box's 36 triangles, 13.9 at eight); more wait on loads:
 // eight (64 registers; 4.63 against 4.67 ms at 1,602 triangles, 7.06 against 7.41 at
-// 33K, 12.65 against 13.59 at 4.2M), but six where those hold the whole image at
-// once, which gains nothing from more and loses what spills cost (72K triangles
-// 64x64x1 226 against 220 us, 100x75x1 269 / 261, 256x256x1 317 / 307).
+// 33K, 12.65 against 13.59 at 4.2M), but six where an image fills those once (split)
+// or twice, which gains little from more and loses what spills cost (72K triangles
+// 64x64x1 226 against 220 us, 100x75x1 269 / 261, 256x256x1 317 / 307; 44K triangles
+// 477x315x1 411 / 396 with the faithful estimator, 560x380x1 711 / 697 with the other).
 //
 // Split: a quarter of the pixels then fills the GPU, the end of the launch is evened
 // out and a tile's rays stay in one SM's L1: mesh 1920x1080x4 12.4 -> 11.6 ms,
@@ -74,9 +76,16 @@ CRG_HD uint32_t few_rays_per_warp(uint64_t n, uint32_t width, uint32_t ntri, boo
 // (327 on a traversal per thread), 64x64x3 532 -> 218 (505), 400x300x2 489 -> 334,
 // 640x480x2 637 -> 626, 1283x721x2 1,164 -> 1,340; six placements 160x120x2 254 -> 143,
 // 256x256x2 353 -> 406; the box 160x120x2 138 -> 86, 256x256x2 162 -> 186.
+//
+// Pixels of a warp: an image of one sample that leaves warps idle lasts as long as its
+// slowest warp, and a warp of fewer pixels is faster: its lanes without a ray test
+// triangles only.  A large scene takes 16, 8 or 4 where the warps then still run at
+// once, against 32 (and a traversal per thread): 11K triangles 80x75x1 with 16 bounces
+// 456 -> 243 us at 4 (346), 480K triangles 254x96x1 529 -> 365 at 8 (495), 200x200x1
+// 642 -> 486 at 16 (546); 380x300x1, too large for 16, 674 against 658.
 struct RenderForm {
     bool split;
-    uint32_t blocks;
+    uint32_t blocks, pixels;
 };
 CRG_HD RenderForm render_form(uint64_t npix, uint32_t spp, uint32_t ntri, bool placed, uint32_t sms) {
     const bool small = ntri < 1024u;
@@ -85,7 +94,10 @@ CRG_HD RenderForm render_form(uint64_t npix, uint32_t spp, uint32_t ntri, bool p
     f.blocks = placed ? 4u : small ? 6u : 8u;
     if (spp >= 4u) f.split = !(small && !placed && npix >= 4u * wave);
     else f.split = spp >= 2u && npix <= (f.blocks == 8u ? 4u : 1u) * 32ull * f.blocks * sms;
-    if (f.blocks == 8u && npix * (f.split ? 4u : 1u) <= wave) f.blocks = 6u;
+    f.pixels = 32u;
+    if (f.blocks == 8u && !f.split)
+        while (f.pixels > 4u && npix * 64u <= wave * f.pixels) f.pixels /= 2u;
+    if (f.blocks == 8u && npix * (f.split ? 4u : 1u) <= (f.split ? wave : 2u * wave)) f.blocks = 6u;
     return f;
 }
 

@@ -20,7 +20,7 @@ def test_small_scene(ctx, orc, size, spp, mode, rr):
 
 @pytest.mark.parametrize("mode,rr", [(1, 3), (0, 0)])
 @pytest.mark.parametrize("spp", [1, 2, 3, 4])
-@pytest.mark.parametrize("size", [(13, 7), (197, 197), (198, 197), (512, 304), (513, 304)])
+@pytest.mark.parametrize("size", [(13, 7), (152, 96), (153, 96), (304, 96), (197, 197), (198, 197), (512, 304), (513, 304)])
 def test_larger_scene(ctx, orc, size, spp, mode, rr):
     sc = scenes.displaced_scene(freq=8)
     st = api.make_settings(size[0], size[1], spp, max_bounces=5, rr_depth=rr, mode=mode, seed=92, aspect=size[0] / size[1])

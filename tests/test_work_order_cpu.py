@@ -18,7 +18,7 @@ extern "C" void sample_share(uint32_t spp, uint32_t parts, uint32_t part, uint32
 }
 extern "C" uint32_t render_form(uint64_t npix, uint32_t spp, uint32_t ntri, uint32_t placed, uint32_t sms) {
     const crg::RenderForm f = crg::render_form(npix, spp, ntri, placed != 0, sms);
-    return f.blocks * 2u + (f.split ? 1u : 0u);
+    return f.pixels << 8 | f.blocks * 2u | (f.split ? 1u : 0u);
 }
 extern "C" uint32_t default_fusion(uint64_t pool, uint64_t largest_chunk, uint32_t host_loop) {
     return crg::default_fusion(pool, largest_chunk, host_loop);
@@ -95,17 +95,25 @@ def test_default_fusion_goes_by_the_pool_and_its_refills(lib):
 def test_render_form_by_samples_pixels_and_scene(lib):
     def form(npix, spp, ntri=5000, placed=0, sms=152):
         v = lib.render_form(C.c_uint64(npix), spp, ntri, placed, sms)
-        return v // 2, bool(v & 1)
+        return (v & 0xFF) // 2, bool(v & 1)
+
+    def pixels(npix, spp, ntri=5000, placed=0, sms=152):
+        return lib.render_form(C.c_uint64(npix), spp, ntri, placed, sms) >> 8
 
     lane = 6 * 152 * 128  # pixels of one wave at a lane each
-    # one sample is never split; a large scene takes six blocks up to a wave, eight above
-    assert [form(n, 1) for n in (1, lane, lane + 1)] == [(6, False), (6, False), (8, False)]
+    # one sample is never split; a large scene takes six blocks up to two waves, eight above
+    assert [form(n, 1) for n in (1, 2 * lane, 2 * lane + 1)] == [(6, False), (6, False), (8, False)]
     assert [form(n, 1, ntri=36) for n in (1, 10 * lane)] == [(6, False)] * 2
     # two and three only where all blocks run at once, four times as many of a large scene
-    assert [form(n, spp) for spp in (2, 3) for n in (4 * 32 * 8 * 152, 4 * 32 * 8 * 152 + 1)] == [(8, True), (8, False)] * 2
+    assert [form(n, spp) for spp in (2, 3) for n in (4 * 32 * 8 * 152, 4 * 32 * 8 * 152 + 1)] == [(8, True), (6, False)] * 2
+    assert form(2 * lane + 1, 3) == (8, False)
     assert [form(n, 2, ntri=36) for n in (32 * 6 * 152, 32 * 6 * 152 + 1)] == [(6, True), (6, False)]
     assert [form(n, 2, placed=1) for n in (32 * 4 * 152, 32 * 4 * 152 + 1)] == [(4, True), (4, False)]
     # four and more: split, but not views of four waves of a small scene without placements
     assert [form(n, 4) for n in (1, lane // 4, lane // 4 + 1, 1 << 31)] == [(6, True), (6, True), (8, True), (8, True)]
     assert [form(n, 4, ntri=36) for n in (4 * lane - 1, 4 * lane)] == [(6, True), (6, False)]
     assert form(4 * lane, 4, ntri=36, placed=1) == (4, True)
+    # pixels of a warp: as few as keep all warps running at once, for a large scene unsplit
+    warps = lane // 32
+    assert [pixels(warps * k + d, 1) for k in (4, 8, 16) for d in (0, 1)] == [4, 8, 8, 16, 16, 32]
+    assert [pixels(1, *a) for a in ((1, 36), (1, 5000, 1), (2, 5000), (4, 5000))] == [32] * 4
