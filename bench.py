@@ -134,18 +134,20 @@ def post_image(w, h):
     return img
 
 
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) from ncu captures on a GB300:
-#   one wavefront frame, per sample: box scene 512x512x64 1,720 B; displaced scene
-#   1920x1080x16 (path pool 4,194,304) 1,097 B;
-#   k_intersect on the soup, per launch of 16,777,216 closest-hit rays: 923.3 MB.
-TRAFFIC_PER_SAMPLE = {"box": 1720.0, "displaced": 1097.0}
-TRAFFIC_SOUP_LAUNCH = 923.3e6
+# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) from ncu captures of the present
+# kernels on a GB300:
+#   one wavefront frame, per sample (profiles/wavefront_traffic.md): box scene 512x512x64 1,601 B;
+#   displaced scene 1920x1080x16 (path pool 4,194,304) 1,262 B;
+#   k_intersect on the soup, per launch of 16,777,216 closest-hit rays: 923.1 MB
+#   (profiles/warp_shared_tests.md).
+TRAFFIC_PER_SAMPLE = {"box": 1601.0, "displaced": 1262.0}
+TRAFFIC_SOUP_LAUNCH = 923.1e6
 
 
 # DRAM bytes per traversed ray (read + write) of the extend kernel, from the displaced-scene
-# iteration capture (profiles/wavefront_displaced_iteration_full.md, build C: 811 MB over one
-# full-queue iteration of a 4,194,304-path pool, one ray per path)
-DRAM_PER_RAY = {"extend": 811.3e6 / 4194304}
+# iteration capture (profiles/warp_shared_tests.md: 751 MB over one full-queue iteration of a
+# 4,194,304-path pool, one ray per path)
+DRAM_PER_RAY = {"extend": 750.9e6 / 4194304}
 
 
 def traffic_dominant(out, stage):
@@ -169,9 +171,9 @@ def traffic_estimate(workload, out, units):
     return None, None
 
 
-# L2 hit rates (lts__t_sector_hit_rate) of the traversal kernels from ncu captures on a GB300
-# (profiles/wavefront_displaced_iteration_full.md, build C; profiles/k_intersect_soup_full.md)
-L2_HIT = {"extend": 0.671, "shadow": 0.671, "soup_closest": 0.880, "soup_any": 0.860}
+# L2 hit rates (lts__t_sector_hit_rate) of the traversal kernels from the same captures
+# (profiles/warp_shared_tests.md)
+L2_HIT = {"extend": 0.577, "shadow": 0.592, "soup_closest": 0.879, "soup_any": 0.872}
 
 
 def stage_roofline(tuned, work, sh_work, stages, node_bytes, peak):
@@ -952,11 +954,11 @@ def main():
                     "peak_kind": peak_kind, "algorithmic_bytes_per_frame": d["algorithmic_bytes"],
                     "stage_ms_per_frame": d["ms"], "l2_hit_rate": L2_HIT.get(st["dominant"]),
                     "l2_hit_rate_source": "ncu lts__t_sector_hit_rate of the same kernel on the displaced scene "
-                                          "(profiles/wavefront_displaced_iteration_full.md)",
+                                          "(profiles/warp_shared_tests.md)",
                     "stage_share": st["share"], "frame": frame}
     elif args.workload == "soup":
         roofline["l2_hit_rate"] = L2_HIT["soup_closest"]
-        roofline["l2_hit_rate_source"] = "ncu capture of the same launch (profiles/k_intersect_soup_full.md)"
+        roofline["l2_hit_rate_source"] = "ncu capture of the same launch (profiles/warp_shared_tests.md)"
     config = workload_config(args.workload, args.form)
     if args.workload == "batch":
         config["samples_per_step"] = units

@@ -128,7 +128,8 @@ struct GradTape {
 // A warp replays its lanes' paths together, as the forward megakernel traces
 // them (box 256x256: forward + loss + adjoint of 32 samples 6.39 -> 5.39 ms with
 // it, 4.85 with the samples split as well; 4 blocks of 128 per SM, 3 / 5 / 6
-// measured 6.44 / 5.56 / 5.81).
+// measured 6.44 / 5.56 / 5.81).  Bound by latency and its FP64 pipe: that is busy 45%
+// of the time, issue 39%, at 24% of the warp slots (3.05 of 4.85 ms; the forward 1.80).
 //
 // Samples from which they are split over a block's warps: 100x80x32 2.92 -> 1.34
 // ms, 256x256x8 1.48 either way, 384x384x4 1.62 -> 1.76.

@@ -51,7 +51,7 @@ constexpr uint32_t kVisitors = 20;
 // One ray per lane, triangle tests shared by the warp, lanes refilled from the
 // block's run of `chunk` rays (dyn_traverse).  The run's counter lies in the
 // block's shared memory, so calls on several streams share nothing.  Bound by
-// instruction issue (75% of cycles) on incoherent rays; 8 blocks of 128 per SM
+// instruction issue (71% of cycles, the ALU pipe 70%) on incoherent rays; 8 blocks of 128 per SM
 // (64 registers).  1M-triangle soup, width 8: 16.8M closest hits 20.97 -> 11.91
 // ms against one thread per ray with its own triangle tests (9.1 lanes active),
 // 5.0M any hits 2.73 -> 1.76 ms against per-lane refill without shared tests.
